@@ -274,17 +274,6 @@ struct FastColArgs {
   T scale;
 };
 
-// Bulk prefetch of [p, p + bytes) into L2 (p and bytes multiples of 16), in chunks
-// issued by the threads of a transform group.
-__device__ __forceinline__ void l2_prefetch_range(const void* p, unsigned bytes, int t, int nthreads) {
-  constexpr unsigned kChunk = 4096;
-  const char* c = static_cast<const char*>(p);
-  for (unsigned off = (unsigned)t * kChunk; off < bytes; off += (unsigned)nthreads * kChunk) {
-    const unsigned n = bytes - off < kChunk ? bytes - off : kChunk;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(c + off), "r"(n) : "memory");
-  }
-}
-
 // Programmatic dependent launch. A step kernel launched with programmatic stream
 // serialisation may start while the kernel before it in the stream is still running:
 // pdl_wait() returns once that kernel has completed and its writes are visible (at

@@ -54,6 +54,10 @@ struct FftDesc {
   int ns[kMaxPass];
   int twoff[kMaxPass];    // offset (complex elements) of the pass twiddles
   int rootoff[kMaxPass];  // offset of the R roots of unity (odd radices > 3), else -1
+  // for the two-buffer engine (pfc_mixed.cuh): butterflies n / R of each pass, and the
+  // multipliers of the divisions by it and by ns (floor(2^32 / d) + 1, 0 for d = 1)
+  int nr[kMaxPass];
+  unsigned mag_nr[kMaxPass], mag_ns[kMaxPass];
 };
 
 // ---------------------------------------------------------------- small DFTs
@@ -184,17 +188,38 @@ template <int R, bool INV, class T> __device__ __forceinline__ void dft(cplx<T>*
   else dft_odd<R, INV>(v, roots);
 }
 
-// Odd-radix DFT with compile-time roots (R = 5 or 7): cos and sin of 2 pi m / R are
-// literal constants (to 20 digits) instead of a table in memory; the same
+// Odd-radix DFT with compile-time roots (R = 5, 7, 11 or 13): cos and sin of 2 pi m / R are
+// literal constants (to 21 digits) instead of a table in memory; the same
 // (s, d)-symmetric evaluation as dft_odd.
 template <int R> __device__ __forceinline__ double root_cos(int m) {
-  if (R == 5) return m == 1 ? 0.30901699437494742410 : -0.80901699437494742410;
-  // R == 7
-  return m == 1 ? 0.62348980185873353053 : m == 2 ? -0.22252093395631440429 : -0.90096886790241912624;
+  if (R == 5) return m == 1 ? 0.309016994374947424102 : -0.809016994374947424102;
+  if (R == 7) return m == 1 ? 0.623489801858733530525 : m == 2 ? -0.222520933956314404289 : -0.900968867902419126236;
+  if (R == 11)
+    return m == 1 ? 0.841253532831181168862
+         : m == 2 ? 0.415415013001886425529
+         : m == 3 ? -0.142314838273285140443
+         : m == 4 ? -0.654860733945285064056 : -0.959492973614497389890;
+  // R == 13
+  return m == 1 ? 0.885456025653209895900
+       : m == 2 ? 0.568064746731155802512
+       : m == 3 ? 0.120536680255323053335
+       : m == 4 ? -0.354604887042535625969
+       : m == 5 ? -0.748510748171101098635 : -0.970941817426052027157;
 }
 template <int R> __device__ __forceinline__ double root_sin(int m) {
-  if (R == 5) return m == 1 ? 0.95105651629515357212 : 0.58778525229247312917;
-  return m == 1 ? 0.78183148246802980871 : m == 2 ? 0.97492791218182360702 : 0.43388373911755812048;
+  if (R == 5) return m == 1 ? 0.951056516295153572116 : 0.587785252292473129169;
+  if (R == 7) return m == 1 ? 0.781831482468029808708 : m == 2 ? 0.974927912181823607018 : 0.433883739117558120475;
+  if (R == 11)
+    return m == 1 ? 0.540640817455597582108
+         : m == 2 ? 0.909631995354518371412
+         : m == 3 ? 0.989821441880932732376
+         : m == 4 ? 0.755749574354258283774 : 0.281732556841429697711;
+  // R == 13
+  return m == 1 ? 0.464723172043768545656
+       : m == 2 ? 0.822983865893656395797
+       : m == 3 ? 0.992708874098053992801
+       : m == 4 ? 0.935016242685414823440
+       : m == 5 ? 0.663122658240795202377 : 0.239315664287557667149;
 }
 template <int R, bool INV, class T> __device__ __forceinline__ void dft_odd_c(cplx<T>* v) {
   constexpr int H = (R - 1) / 2;

@@ -1,6 +1,6 @@
 // Definitions of GenericInst (pfc_registry.h): included by the .cu file of each precision.
 #pragma once
-#include "pfc_kernels.cuh"
+#include "pfc_mixed.cuh"
 #include "pfc_registry.h"
 
 namespace pfc {
@@ -10,54 +10,40 @@ namespace generic_detail {
 // The nonlinearity only matters in the step and reduce modes; other modes use the std instance.
 template <int MODE> constexpr bool row_uses_model() { return MODE == kRowStep || MODE == kRowReduce; }
 
+template <class T, int MODE, int MODEL>
+void* pick_row_model(int rset) {
+  switch (rset) {
+    case kRadixPow2: return (void*)mixed_row_kernel<T, MODE, MODEL, kRadixPow2>;
+    case kRadixSmall: return (void*)mixed_row_kernel<T, MODE, MODEL, kRadixSmall>;
+    case kRadixAll: return (void*)mixed_row_kernel<T, MODE, MODEL, kRadixAll>;
+    case kRadixPow2Big: return (void*)row_kernel<T, MODE, MODEL, kRadixPow2, 1024>;
+    case kRadixSmallBig: return (void*)row_kernel<T, MODE, MODEL, kRadixSmall, 1024>;
+    default: return nullptr;
+  }
+}
+
 template <class T, int MODE>
 void* pick_row(int model, int rset) {
-  const bool log = row_uses_model<MODE>() && model == kModelLog;
-  if (rset == kRadixAllDense) {
-    if constexpr (sizeof(T) == 4 && MODE == kRowStep)
-      return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixAll, 256, 2>
-                 : (void*)row_kernel<T, MODE, kModelStd, kRadixAll, 256, 2>;
-    rset = kRadixAll;
-  }
-  if (rset == kRadixSmallDense) {
-    if constexpr (sizeof(T) == 4 && MODE == kRowStep)
-      return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixSmall, 256, 2>
-                 : (void*)row_kernel<T, MODE, kModelStd, kRadixSmall, 256, 2>;
-    rset = kRadixSmall;
-  }
-  if (rset == kRadixSmall)
-    return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixSmall, 256>
-               : (void*)row_kernel<T, MODE, kModelStd, kRadixSmall, 256>;
-  if (rset == kRadixSmallBig)
-    return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixSmall, 1024>
-               : (void*)row_kernel<T, MODE, kModelStd, kRadixSmall, 1024>;
-  if (rset == kRadixPow2Big)
-    return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixPow2, 1024>
-               : (void*)row_kernel<T, MODE, kModelStd, kRadixPow2, 1024>;
-  if (rset == kRadixPow2)
-    return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixPow2, 256>
-               : (void*)row_kernel<T, MODE, kModelStd, kRadixPow2, 256>;
-  return log ? (void*)row_kernel<T, MODE, kModelLog, kRadixAll, 256>
-             : (void*)row_kernel<T, MODE, kModelStd, kRadixAll, 256>;
+  if constexpr (row_uses_model<MODE>())
+    if (model == kModelLog) return pick_row_model<T, MODE, kModelLog>(rset);
+  return pick_row_model<T, MODE, kModelStd>(rset);
 }
 
 template <class T, int MODE>
 void* pick_col(int rset) {
-  if (rset == kRadixAllDense) {
-    if constexpr (sizeof(T) == 4 && MODE == kColStep) return (void*)col_kernel<T, MODE, kRadixAll, 256, 2>;
-    rset = kRadixAll;
+  // (the Parseval and export modes transform nothing)
+  if constexpr (MODE == kColParseval || MODE == kColExport) {
+    return (void*)col_kernel<T, MODE, kRadixPow2, 256>;
+  } else {
+    switch (rset) {
+      case kRadixPow2: return (void*)mixed_col_kernel<T, MODE, kRadixPow2>;
+      case kRadixSmall: return (void*)mixed_col_kernel<T, MODE, kRadixSmall>;
+      case kRadixAll: return (void*)mixed_col_kernel<T, MODE, kRadixAll>;
+      case kRadixPow2Big: return (void*)col_kernel<T, MODE, kRadixPow2, 1024>;
+      case kRadixSmallBig: return (void*)col_kernel<T, MODE, kRadixSmall, 1024>;
+      default: return nullptr;
+    }
   }
-  if (rset == kRadixSmallDense) {
-    if constexpr (sizeof(T) == 4 && MODE == kColStep) return (void*)col_kernel<T, MODE, kRadixSmall, 256, 2>;
-    rset = kRadixSmall;
-  }
-  if (rset == kRadixSmall && MODE != kColParseval && MODE != kColExport) return (void*)col_kernel<T, MODE, kRadixSmall, 256>;
-  if (rset == kRadixPow2Big) return (void*)col_kernel<T, MODE, kRadixPow2, 1024>;
-  if (rset == kRadixSmallBig)   // (the Parseval and export modes transform nothing)
-    return (MODE == kColParseval || MODE == kColExport) ? (void*)col_kernel<T, MODE, kRadixPow2, 1024>
-                                                        : (void*)col_kernel<T, MODE, kRadixSmall, 1024>;
-  if (MODE == kColParseval || MODE == kColExport || rset == kRadixPow2) return (void*)col_kernel<T, MODE, kRadixPow2, 256>;
-  return (void*)col_kernel<T, MODE, kRadixAll, 256>;
 }
 
 }  // namespace generic_detail

@@ -164,10 +164,18 @@ struct BatchBufs {
   const double* scal;   // deviation-form scalars
 };
 
+// What a batched reduction takes from each plan besides its buffers.
+struct BatchReduce {
+  double epsilon, beta, q0, fx, fy;   // fx = 1/(nx dx), fy = 1/(ny dy)
+  double lmu0, lf0;
+  int* status;
+};
+
 template <class T>
 struct RowArgs {
   int nx, ny, m, rows, tpf, ld;
-  FftDesc fft;
+  int rows_log2;            // two-buffer engine: rows = 1 << rows_log2
+  FftDesc fft, fft_b;       // the transform; the same radices in reverse order
   const cplx<T>* tw;
   const cplx<T>* rtw;       // exp(-2 pi i k / nx), k < m
   const cplx<T>* in;        // packed spectra [kx][y]
@@ -180,7 +188,9 @@ struct RowArgs {
   double* minmax;           // step mode, FP64 form: per-CTA (min, max) of the field, or null
   int clamp;
   double g, min_phi, min_log, epsilon;
-  const BatchBufs* batch;   // step mode of a batch: per-plan W, V and scalars at [blockIdx.y]
+  const BatchBufs* batch;   // step or reduce mode of a batch: per-plan W, V and scalars at [blockIdx.y]
+  const BatchReduce* red;   // reduce mode of a batch: the plans' parameters
+  int partials_stride;      //   and the doubles between two plans' partials
 };
 
 // The spectral state and the update n_hat' = n_hat + (A - 1) n_hat + Bg N_hat.
@@ -193,7 +203,7 @@ struct RowArgs {
 template <class T>
 struct ColArgs {
   int nx, ny, m, cols, tpf, ld, nyh;
-  FftDesc fft;
+  FftDesc fft, fft_b;           // the transform; the same radices in reverse order
   const cplx<T>* tw;
   const cplx<T>* in;            // V (step/init/combine)
   const void* sin;              // n_hat (parseval/export): complex128, or hi (FP32 form)
@@ -215,7 +225,9 @@ struct ColArgs {
   double fx, fy;                // 1/(nx dx), 1/(ny dy): k = 2 pi idx f
   double beta, q0, epsilon, w;  // L_mu, L_f, Gaussian width
   const double* scal;           // device scalar block (export adds the deviation-form DC)
-  const BatchBufs* batch;       // step mode of a batch: per-plan buffers at [blockIdx.y]
+  const BatchBufs* batch;       // step or Parseval mode of a batch: per-plan buffers at [blockIdx.y]
+  const BatchReduce* red;       // Parseval mode of a batch: the plans' parameters
+  int partials_stride;          //   and the doubles between two plans' partials
 };
 
 // Element i of a spectral state (hi + lo in the FP32 form when with_lo).
@@ -272,7 +284,39 @@ __device__ __forceinline__ double ksq(int kx, int ky, int ny, double fx, double 
   return kxp * kxp + kyp * kyp;
 }
 
-// ---------------------------------------------------------------- row kernel
+// Bulk prefetch of [p, p + bytes) into L2 (p and bytes multiples of 16), in chunks
+// issued by `nthreads` threads, this one the t-th.
+__device__ __forceinline__ void l2_prefetch_range(const void* p, unsigned bytes, int t, int nthreads) {
+  constexpr unsigned kChunk = 4096;
+  const char* c = static_cast<const char*>(p);
+  for (unsigned off = (unsigned)t * kChunk; off < bytes; off += (unsigned)nthreads * kChunk) {
+    const unsigned n = bytes - off < kChunk ? bytes - off : kChunk;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(c + off), "r"(n) : "memory");
+  }
+}
+
+// One site's terms of the reductions: the raw value, the free-energy polynomial and the
+// nonlinear mu of n = mean + v.
+template <int MODEL>
+__device__ __forceinline__ void row_reduce_add(KSum* acc, double mean, double v, double eps, double g, int clamp,
+                                               double min_phi, double min_log) {
+  const double n = mean + v;
+  const double n2 = n * n;
+  double fpoly = (eps / 2.0) * n2 + (g / 3.0) * (n2 * n) + (1 / 4.0) * (n2 * n2);
+  double nl = g * n2 + n2 * n;
+  if (MODEL == kModelLog) {
+    const double lg = log(n);
+    fpoly = n * lg + fpoly;
+    nl += (clamp && !(n > min_phi)) ? min_log : lg;
+  }
+  ksum_add(acc[0], v);
+  ksum_add(acc[1], fpoly);
+  ksum_add(acc[2], nl);
+}
+
+// ---------------------------------------------------------------- row kernel (one buffer)
+// The one-buffer kernels below serve the transforms whose two buffers (pfc_mixed.cuh) do not
+// fit an SM's shared memory.
 // rows transforms of length m per CTA, tpf threads each; smem = rows * ld complex.
 template <class T, int MODE, int MODEL, int RSET, int LB = 256, int MINB = 1>
 __global__ void __launch_bounds__(LB, MINB) row_kernel(RowArgs<T> a) {
@@ -416,20 +460,7 @@ __global__ void __launch_bounds__(LB, MINB) row_kernel(RowArgs<T> a) {
         const cplx<T> z = buf[j];
         const double vv[2] = {(double)z.x, (double)z.y};
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const double n = mean + vv[h];
-          const double n2 = n * n;
-          double fpoly = (eps / 2.0) * n2 + (g / 3.0) * (n2 * n) + (1 / 4.0) * (n2 * n2);
-          double nl = g * n2 + n2 * n;
-          if (MODEL == kModelLog) {
-            const double ln = (a.clamp && !(n > a.min_phi)) ? a.min_log : log(n);
-            fpoly = n * log(n) + fpoly;
-            nl += ln;
-          }
-          ksum_add(acc[0], vv[h]);
-          ksum_add(acc[1], fpoly);
-          ksum_add(acc[2], nl);
-        }
+        for (int h = 0; h < 2; ++h) row_reduce_add<MODEL>(acc, mean, vv[h], eps, g, a.clamp, a.min_phi, a.min_log);
       }
     }
     block_reduce_store<3>(acc, a.partials + 6 * blockIdx.x);
@@ -441,6 +472,23 @@ template <class T>
 __device__ __forceinline__ void unpack_pair(cplx<T> pk, cplx<T> pkp, cplx<T>& h0, cplx<T>& hm) {
   h0 = T(0.5) * (pk + conj(pkp));
   hm = T(0.5) * rot4<false>(pk - conj(pkp));
+}
+
+// Multipliers of n_hat and N_hat at (kx, ky) in the combine modes: mu_hat = L_mu n_hat + N_hat
+// (optionally Gaussian-filtered), G n_hat, N_hat or n_hat.
+template <class T>
+__device__ __forceinline__ void col_combine_factors(const ColArgs<T>& a, int kx, int ky, double& mn, double& mq) {
+  const double q2 = a.q0 * a.q0;
+  const double k2 = ksq(kx, ky, a.ny, a.fx, a.fy);
+  const double lmu = a.beta * (q2 - k2) * (q2 - k2) + a.epsilon;
+  const double gs = exp(-k2 * a.w * a.w / 2);
+  switch (a.combine) {
+    case kCombineMu: mn = lmu; mq = 1.0; break;
+    case kCombineLocalMu: mn = gs * lmu; mq = gs; break;
+    case kCombineLocalN: mn = gs; mq = 0.0; break;
+    case kCombineNonlin: mn = 0.0; mq = 1.0; break;
+    default: mn = 1.0; mq = 0.0; break;
+  }
 }
 
 // cols transforms of length ny per CTA, tpf threads each; smem = cols * ld complex.
@@ -478,6 +526,15 @@ __global__ void __launch_bounds__(LB, MINB) col_kernel(ColArgs<T> a) {
   if (MODE == kColParseval || MODE == kColExport) {
     // no transform: direct pass over n_hat
     KSum acc[1] = {{0.0, 0.0}};
+    double* partials = a.partials;
+    if (MODE == kColParseval && a.batch) {
+      const BatchBufs& bb = a.batch[blockIdx.y];
+      const BatchReduce& br = a.red[blockIdx.y];
+      a.sin = bb.nin;
+      a.sin_lo = static_cast<const cplx<float>*>(bb.nin_lo);
+      a.beta = br.beta; a.q0 = br.q0; a.fx = br.fx; a.fy = br.fy;
+      partials += (size_t)blockIdx.y * a.partials_stride;
+    }
     if (valid) {
       const size_t cb = (size_t)kx * ny;
       for (int ky = lt; ky < ny; ky += tpf) {
@@ -511,7 +568,7 @@ __global__ void __launch_bounds__(LB, MINB) col_kernel(ColArgs<T> a) {
         }
       }
     }
-    if (MODE == kColParseval) block_reduce_store<1>(acc, a.partials + 2 * blockIdx.x);
+    if (MODE == kColParseval) block_reduce_store<1>(acc, partials + 2 * blockIdx.x);
     return;
   }
 
@@ -626,24 +683,11 @@ __global__ void __launch_bounds__(LB, MINB) col_kernel(ColArgs<T> a) {
     // mu_hat = L_mu n_hat + N_hat (optionally Gaussian-filtered), or G n_hat, or N_hat
     if (valid) {
       const size_t cb = (size_t)kx * ny;
-      const double q2 = a.q0 * a.q0;
       for (int ky = lt; ky <= ny / 2; ky += tpf) {
         const int kyp = ky == 0 ? 0 : ny - ky;
         // multipliers for n_hat and N_hat at (kx, ky) and, for the packed column, (m, ky)
         double mn[2], mq[2];
-        for (int h = 0; h < (kx == 0 ? 2 : 1); ++h) {
-          const int kxx = (h == 0) ? kx : m;
-          const double k2 = ksq(kxx, ky, ny, a.fx, a.fy);
-          const double lmu = a.beta * (q2 - k2) * (q2 - k2) + a.epsilon;
-          const double gs = exp(-k2 * a.w * a.w / 2);
-          switch (a.combine) {
-            case kCombineMu: mn[h] = lmu; mq[h] = 1.0; break;
-            case kCombineLocalMu: mn[h] = gs * lmu; mq[h] = gs; break;
-            case kCombineLocalN: mn[h] = gs; mq[h] = 0.0; break;
-            case kCombineNonlin: mn[h] = 0.0; mq[h] = 1.0; break;
-            default: mn[h] = 1.0; mq[h] = 0.0; break;
-          }
-        }
+        for (int h = 0; h < (kx == 0 ? 2 : 1); ++h) col_combine_factors(a, h == 0 ? kx : m, ky, mn[h], mq[h]);
         const cplx<double> pk = state_ld<T>(a_nin, a_nin_lo, cb + ky, true);
         const cplx<double> pkp = state_ld<T>(a_nin, a_nin_lo, cb + kyp, true);
         cplx<double> qk = mk(0.0, 0.0), qkp = qk;

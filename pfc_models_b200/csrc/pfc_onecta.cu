@@ -7,103 +7,34 @@
 // buffers and the spectral state) and runs `nsteps` steps in a loop, so a block of steps
 // is one launch; a batch of plans is one launch with one CTA per plan.
 //
-// Each step runs the same device functions, with the same arguments and in the same order,
-// as row_kernel<kRowStep> followed by col_kernel<kColStep> (pfc_kernels.cuh): the packed
-// inverse real transform of the rows, the nonlinearity, the forward real transform, the
-// column transform, the ETD1 update n_hat' = n_hat + (A - 1) n_hat + Bg N_hat and the
-// inverse column transform. On the last step of a launch it leaves in global memory what
+// Each step runs the passes of mixed_row_kernel<kRowStep> followed by those of
+// mixed_col_kernel<kColStep> (pfc_mixed.cuh) with the same arithmetic, every butterfly of all
+// rows (or columns) dealt to the CTA's threads. What bounds a step is the chain of its phases,
+// each a shared-memory read, a short dependent FP64 DFT and a barrier, so here the
+// real-packing twiddles too are applied where the next phase reads: a cell whose sides need
+// two passes each takes 6 phases and barriers a step (16 before), 28 x 24 log cells
+// 8.0 -> 6.4 us a step. On the last step of a launch the kernel leaves in global memory what
 // the two-kernel step leaves: V (the nonlinear spectrum of the state the step started
 // from), that state, the new state and W (the new state's inverse column transforms).
-#include "pfc_kernels.cuh"
+#include "pfc_mixed.cuh"
 #include "pfc_registry.h"
 
 namespace pfc {
 
 namespace {
 
-// One Stockham pass from src to dst with one butterfly per thread at a time: the loads,
-// twiddles, DFT and output positions of stockham_pass (pfc_fft.cuh), out of place, so a
-// thread holds R values instead of all its butterflies and the pass needs one barrier.
-template <int R, bool INV>
-__device__ __forceinline__ void pass_oop(PadBuf<double> src, PadBuf<double> dst, int n, int ns,
-                                         const cplx<double>* __restrict__ tw, const cplx<double>* __restrict__ roots,
-                                         int lt, int tpf) {
-  const int nr = n / R;
-  for (int j = lt; j < nr; j += tpf) {
-    cplx<double> v[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = src[j + q * nr];
-    const int k = j % ns;
-    if (k != 0) {
-      const cplx<double>* w = tw + k;   // table [q - 1][k]
-#pragma unroll
-      for (int q = 1; q < R; ++q) {
-        cplx<double> t = w[(q - 1) * ns];
-        if (INV) t.y = -t.y;
-        v[q] = cmul(v[q], t);
-      }
-    }
-    dft<R, INV>(v, roots);
-    const int base = (j - k) * R + k;
-#pragma unroll
-    for (int q = 0; q < R; ++q) dst[base + q * ns] = v[q];
-  }
-  __syncthreads();
-}
-
-// Every pass of d, alternating between buffers a and b (every thread of the CTA calls
-// this); the result is in b when the pass count is odd, else in a. Out of line: the step
-// calls each direction twice, and one copy of the butterflies per direction keeps the
-// kernel's code small enough for the instruction cache.
-template <bool INV, int RSET>
-__device__ __noinline__ void fft_oop(PadBuf<double> a, PadBuf<double> b, const FftDesc& d,
-                                        const cplx<double>* __restrict__ twbase, int lt, int tpf) {
-  PadBuf<double> src = a, dst = b;
-  for (int p = 0; p < d.npass; ++p) {
-    const cplx<double>* tw = twbase + d.twoff[p];
-    const cplx<double>* roots = d.rootoff[p] >= 0 ? twbase + d.rootoff[p] : nullptr;
-    const int ns = d.ns[p];
-    switch (d.radix[p]) {
-      case 2: pass_oop<2, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-      case 4: pass_oop<4, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-      case 8: pass_oop<8, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-      case 16: pass_oop<16, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-      default:
-        if constexpr (RSET != kRadixPow2) {
-          switch (d.radix[p]) {
-            case 3: pass_oop<3, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-            case 5: pass_oop<5, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-            case 7: pass_oop<7, INV>(src, dst, d.n, ns, tw, roots, lt, tpf); break;
-            default:
-              if constexpr (RSET == kRadixAll) {
-                if (d.radix[p] == 11) pass_oop<11, INV>(src, dst, d.n, ns, tw, roots, lt, tpf);
-                else if (d.radix[p] == 13) pass_oop<13, INV>(src, dst, d.n, ns, tw, roots, lt, tpf);
-              }
-              break;
-          }
-        }
-        break;
-    }
-    const PadBuf<double> t = src;
-    src = dst;
-    dst = t;
-  }
-}
-
 // MINB 1: all registers for one CTA per SM (single plans, small batches); MINB 2: two
-// CTAs per SM (batches with more plans than SMs; a few spilled values).
+// CTAs per SM (batches with more plans than SMs).
 template <int MODEL, int RSET, int MINB>
 __global__ void __launch_bounds__(kOneCtaMaxThreads, MINB) onecta_step_kernel(RowArgs<double> ra, ColArgs<double> ca,
                                                                          const BatchBufs* table, long long nsteps) {
   using T = double;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int m = ra.m, ny = ra.ny, ldr = ra.ld, ldc = ca.ld, nyh = ca.nyh;
-  const int spec = m * ny;
-  cplx<T>* R = reinterpret_cast<cplx<T>*>(smem_raw);   // ny row buffers of ldr
-  cplx<T>* R2 = R + (size_t)ny * ldr;                     // their pass partners
-  cplx<T>* C = R2 + (size_t)ny * ldr;                     // m column buffers of ldc
-  cplx<T>* C2 = C + (size_t)m * ldc;                      // their pass partners
-  cplx<T>* S = C2 + (size_t)m * ldc;                      // n_hat, packed [kx][y]
+  const int spec = m * ny, half = max(ny * ldr, m * ldc);
+  cplx<T>* src = reinterpret_cast<cplx<T>*>(smem_raw);   // ny row buffers of ldr, or m column buffers of ldc
+  cplx<T>* dst = src + half;
+  cplx<T>* S = dst + half;                               // n_hat, packed [kx][y]
   const BatchBufs& bb = table[blockIdx.x];
   cplx<T>* W = static_cast<cplx<T>*>(const_cast<void*>(bb.w));
   cplx<T>* V = static_cast<cplx<T>*>(bb.v);
@@ -113,143 +44,158 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, MINB) onecta_step_kernel(Ro
 
   for (int i = tid; i < spec; i += nth) {
     const int kx = i / ny, y = i - kx * ny;
-    C[kx * ldc + generic_pad(y)] = W[i];
+    src[kx * ldc + generic_pad(y)] = W[i];
     S[i] = P[0][i];
   }
-  // Roles: thread tid works on row tid / tpf_r and on column tid / tpf_c. A thread
-  // without a row (or column) gets a lane index past every butterfly and pair loop, so
-  // it touches no buffer there but still reaches every barrier of the transforms.
-  const int tr = ra.tpf, tc = ca.tpf;
-  const int fr = tid / tr, fc = tid / tc;
-  const bool row_on = fr < ny, col_on = fc < m;
-  constexpr int kIdle = 1 << 20;
-  const int ltr = row_on ? tid - fr * tr : kIdle;
-  const int ltc = col_on ? tid - fc * tc : kIdle;
-  const PadBuf<T> rbuf{R + (size_t)(row_on ? fr : 0) * ldr}, rbuf2{R2 + (size_t)(row_on ? fr : 0) * ldr};
-  const PadBuf<T> cbuf{C + (size_t)(col_on ? fc : 0) * ldc}, cbuf2{C2 + (size_t)(col_on ? fc : 0) * ldc};
-  const int kx = col_on ? fc : 0;
-  const T s = (T)ca.scale;
-  const FftDesc& rfft = ra.fft;
-  const FftDesc& cfft = ca.fft;
-  // where a transform's result lands: the partner buffer after an odd pass count; an
-  // inverse and a forward transform together always end in the main buffer
-  const PadBuf<T> xr = (rfft.npass & 1) ? rbuf2 : rbuf, xr2 = (rfft.npass & 1) ? rbuf : rbuf2;
-  const PadBuf<T> xc = (cfft.npass & 1) ? cbuf2 : cbuf, xc2 = (cfft.npass & 1) ? cbuf : cbuf2;
   __syncthreads();
+  const T s = (T)ca.scale;
+  const FftDesc &ra_a = ra.fft, &ra_b = ra.fft_b, &ca_a = ca.fft, &ca_b = ca.fft_b;
+  const int npr = ra_a.npass, npc = ca_a.npass;
+
+  auto ld_r = [&](int f, int i) { return src[f * ldr + generic_pad(i)]; };
+  auto st_r = [&](int f, int i, cplx<T> v) { dst[f * ldr + generic_pad(i)] = v; };
+  auto ld_c = [&](int f, int i) { return src[f * ldc + generic_pad(i)]; };
+  auto st_c = [&](int f, int i, cplx<T> v) { dst[f * ldc + generic_pad(i)] = v; };
+  auto flip = [&]() {
+    __syncthreads();
+    cplx<T>* t = src;
+    src = dst;
+    dst = t;
+  };
+  // row y's element k of the inverse transform's input, from the columns of W
+  auto ld_pre = [&](int y, int k) {
+    if (k == 0) return real_dc(src[generic_pad(y)]);
+    const int kk = min(k, m - k);
+    cplx<T> zk, zm;
+    real_pre(src[kk * ldc + generic_pad(y)], src[(m - kk) * ldc + generic_pad(y)], ra.rtw[kk], zk, zm);
+    return k == kk ? zk : zm;
+  };
 
   for (long long step = 0; step < nsteps; ++step) {
     const bool last = step == nsteps - 1;
-    // ---- row pass (row_kernel<kRowStep>)
-    for (int i = tid; i < spec; i += nth) {
-      const int c = i / ny, y = i - c * ny;
-      R[y * ldr + generic_pad(c)] = C[c * ldc + generic_pad(y)];
-    }
-    __syncthreads();
-    for (int k = ltr; k <= m / 2; k += tr) {
-      if (k == 0) {
-        const cplx<T> p = rbuf[0];
-        rbuf[0] = mk(p.x + p.y, p.x - p.y);
-      } else {
-        const int kk = m - k;
-        const cplx<T> xk = rbuf[k], xm = rbuf[kk];
-        const cplx<T> sm = xk + conj(xm), d = xk - conj(xm);
-        const cplx<T> u = mul_i(cmul(conj(ra.rtw[k]), d));
-        rbuf[k] = sm + u;
-        if (kk != k) rbuf[kk] = conj(sm - u);
-      }
-    }
-    __syncthreads();
-    fft_oop<true, RSET>(rbuf, rbuf2, rfft, ra.tw, ltr, tr);
-    for (int j = ltr; j < m; j += tr) {
-      const cplx<T> z = xr[j];
-      xr[j] = mk((T)nonlin_plain<MODEL>((double)z.x, ra.g, ra.clamp, ra.min_phi, ra.min_log),
-                   (T)nonlin_plain<MODEL>((double)z.y, ra.g, ra.clamp, ra.min_phi, ra.min_log));
-    }
-    __syncthreads();
-    fft_oop<false, RSET>(xr, xr2, rfft, ra.tw, ltr, tr);
-    for (int k = ltr; k <= m / 2; k += tr) {
-      if (k == 0) {
-        const cplx<T> z = rbuf[0];
-        rbuf[0] = mk(z.x + z.y, z.x - z.y);
-      } else {
-        const int kk = m - k;
-        const cplx<T> zk = rbuf[k], zm = rbuf[kk];
-        const cplx<T> e = T(0.5) * (zk + conj(zm));
-        const cplx<T> o = T(0.5) * rot4<false>(zk - conj(zm));
-        const cplx<T> t = cmul(ra.rtw[k], o);
-        rbuf[k] = e + t;
-        if (kk != k) rbuf[kk] = conj(e - t);
-      }
-    }
-    __syncthreads();
-    // ---- column pass (col_kernel<kColStep>)
-    for (int i = tid; i < spec; i += nth) {
-      const int c = i / ny, y = i - c * ny;
-      const cplx<T> v = R[y * ldr + generic_pad(c)];
-      C[c * ldc + generic_pad(y)] = v;
-      if (last) V[i] = v;
-    }
-    if (last)   // the state this step starts from, in its ping-pong buffer
-      for (int i = tid; i < spec; i += nth) P[step & 1][i] = S[i];
-    __syncthreads();
-    fft_oop<false, RSET>(cbuf, cbuf2, cfft, ca.tw, ltc, tc);
-    if (col_on && kx == 0) {
-      for (int ky = ltc; ky <= ny / 2; ky += tc) {
-        const int kyp = ky == 0 ? 0 : ny - ky;
-        const cplx<T> qkt = xc[ky], qkpt = xc[kyp];
-        const cplx<double> qk = mk((double)qkt.x, (double)qkt.y), qkp = mk((double)qkpt.x, (double)qkpt.y);
-        const cplx<double> c0v = coef[ky];
-        const cplx<double> cMv = coef[(size_t)m * nyh + ky];
-        const cplx<double> pk = S[ky];
-        const cplx<double> pkp = S[kyp];
-        cplx<double> h0, hm, g0, gm;
-        unpack_pair(pk, pkp, h0, hm);
-        unpack_pair(qk, qkp, g0, gm);
-        const cplx<double> h0n = h0 + c0v.x * h0 + c0v.y * g0;
-        const cplx<double> hmn = hm + cMv.x * hm + cMv.y * gm;
-        const cplx<double> ok = h0n + mul_i(hmn);
-        const cplx<double> okp = conj(h0n) + mul_i(conj(hmn));
-        S[ky] = ok;
-        xc[ky] = mk((T)ok.x, (T)ok.y);
-        if (kyp != ky) {
-          S[kyp] = okp;
-          xc[kyp] = mk((T)okp.x, (T)okp.y);
-        }
-      }
-    } else if (col_on) {
-      const size_t cb = (size_t)kx * ny;
-      for (int ky = ltc; ky <= ny / 2; ky += tc) {
-        const int kyp = ky == 0 ? 0 : ny - ky;
-        const cplx<T> cw = coef[(size_t)kx * nyh + ky];
-        const cplx<T> ph = S[cb + ky], pph = S[cb + kyp];
-        const cplx<T> qkt = xc[ky], qkpt = xc[kyp];
-        const cplx<double> qk = mk((double)qkt.x, (double)qkt.y), qkp = mk((double)qkpt.x, (double)qkpt.y);
-        const cplx<double> c = mk((double)cw.x, (double)cw.y);
-        const cplx<double> pk = mk((double)ph.x, (double)ph.y), pkp = mk((double)pph.x, (double)pph.y);
-        const cplx<double> ok = pk + c.x * pk + c.y * qk;
-        const cplx<double> okp = pkp + c.x * pkp + c.y * qkp;
-        S[cb + ky] = ok;
-        xc[ky] = mk((T)ok.x, (T)ok.y);
-        if (kyp != ky) {
-          S[cb + kyp] = okp;
-          xc[kyp] = mk((T)okp.x, (T)okp.y);
-        }
-      }
-    }
-    __syncthreads();
-    fft_oop<true, RSET>(xc, xc2, cfft, ca.tw, ltc, tc);
-    for (int ky = ltc; ky < ny; ky += tc) {
-      const cplx<T> v = cbuf[ky];
-      cbuf[ky] = mk(s * v.x, s * v.y);
-    }
-    __syncthreads();
-    if (last) {
+    // ---- row pass
+    if (npr == 1) {
       for (int i = tid; i < spec; i += nth) {
-        const int c = i / ny, y = i - c * ny;
-        P[(step + 1) & 1][i] = S[i];
-        W[i] = C[c * ldc + generic_pad(y)];
+        const int y = i / m, k = i - y * m;
+        st_r(y, k, ld_pre(y, k));
+      }
+      flip();
+    } else {
+      mixed_pass<true, RSET, T>(ra_a, 0, ny, ra.tw, ld_pre, st_r);
+      flip();
+      for (int p = 1; p < npr - 1; ++p) {
+        mixed_pass<true, RSET, T>(ra_a, p, ny, ra.tw, ld_r, st_r);
+        flip();
       }
     }
+    struct Nonlin {
+      struct Aux {};
+      const RowArgs<double>* a;
+      __device__ __forceinline__ Aux load(int, int) const { return Aux{}; }
+      __device__ __forceinline__ void apply(int, int, Aux, cplx<T>& z) const {
+        z = mk((T)nonlin_plain<MODEL>((double)z.x, a->g, a->clamp, a->min_phi, a->min_log),
+               (T)nonlin_plain<MODEL>((double)z.y, a->g, a->clamp, a->min_phi, a->min_log));
+      }
+    } fn{&ra};
+    mixed_switch<RSET, T>(ra_a.radix[npr - 1], [&](auto r) {
+      mixed_mid_items<decltype(r)::value, true, T>(ra_a, 0, ny, ra.tw, ld_r, fn, st_r);
+    });
+    flip();
+    for (int p = 1; p < npr; ++p) {
+      mixed_pass<false, RSET, T>(ra_b, p, ny, ra.tw, ld_r, st_r);
+      flip();
+    }
+    // ---- column pass: V[kx][y] from the rows' transforms
+    auto ld_post = [&](int kx, int y) {
+      const cplx<T>* row = src + y * ldr;
+      cplx<T> v;
+      if (kx == 0) {
+        v = real_dc(row[0]);
+      } else {
+        const int kk = min(kx, m - kx);
+        cplx<T> yk, ym;
+        real_post(row[generic_pad(kk)], row[generic_pad(m - kk)], ra.rtw[kk], yk, ym);
+        v = kx == kk ? yk : ym;
+      }
+      if (last) V[kx * ny + y] = v;
+      return v;
+    };
+    if (npc == 1) {
+      for (int i = tid; i < spec; i += nth) {
+        const int kx = i / ny, y = i - kx * ny;
+        st_c(kx, y, ld_post(kx, y));
+      }
+      flip();
+    } else {
+      mixed_pass<false, RSET, T>(ca_a, 0, m, ca.tw, ld_post, st_c);
+      flip();
+      for (int p = 1; p < npc - 1; ++p) {
+        mixed_pass<false, RSET, T>(ca_a, p, m, ca.tw, ld_c, st_c);
+        flip();
+      }
+    }
+    // the last step leaves the state it starts from and the new one in global memory
+    cplx<T>* p_old = last ? P[step & 1] : nullptr;
+    cplx<T>* p_new = P[(step + 1) & 1];
+    struct Update {
+      struct Aux {
+        cplx<T> c, p;
+      };
+      const cplx<T>* coef;
+      cplx<T> *S, *p_old, *p_new;
+      int ny, nyh;
+      __device__ __forceinline__ Aux load(int kx, int ky) const {
+        return Aux{coef[kx * nyh + (ky <= ny / 2 ? ky : ny - ky)], S[kx * ny + ky]};
+      }
+      __device__ __forceinline__ void put(int i, cplx<T> was, cplx<T> now) const {
+        S[i] = now;
+        if (p_old) {
+          p_old[i] = was;
+          p_new[i] = now;
+        }
+      }
+      __device__ __forceinline__ void apply(int kx, int ky, const Aux& x, cplx<T>& v) const {
+        const cplx<double> o = x.p + x.c.x * x.p + x.c.y * v;
+        put(kx * ny + ky, x.p, o);
+        v = o;
+      }
+    } up{coef, S, p_old, p_new, ny, nyh};
+    mixed_switch<RSET, T>(ca_a.radix[npc - 1], [&](auto r) {
+      constexpr int R = decltype(r)::value;
+      mixed_mid_items<R, false, T>(ca_a, 1, m, ca.tw, ld_c, up, st_c);
+      mixed_mid_paired<R, false, T>(ca_a, ca.tw, ld_c, [&](int ky, int kyp, cplx<T>& v, cplx<T>& vp) {
+        const int kh = min(ky, kyp);
+        const cplx<T> pk = S[ky], pkp = S[kyp];
+        cplx<T> ok, okp;
+        packed_update(pk, pkp, v, vp, coef[kh], coef[m * nyh + kh], nullptr, nullptr, ok, okp);
+        up.put(ky, pk, ok);
+        v = ok;
+        if (kyp != ky) {
+          up.put(kyp, pkp, okp);
+          vp = okp;
+        }
+      }, st_c);
+    });
+    flip();
+    // ---- inverse columns: W
+    auto st_w = [&](int kx, int y, cplx<T> v) {
+      const cplx<T> w = mk(s * v.x, s * v.y);
+      dst[kx * ldc + generic_pad(y)] = w;
+      if (last) W[kx * ny + y] = w;
+    };
+    if (npc == 1) {
+      for (int i = tid; i < spec; i += nth) {
+        const int kx = i / ny, y = i - kx * ny;
+        st_w(kx, y, ld_c(kx, y));
+      }
+    } else {
+      for (int p = 1; p < npc - 1; ++p) {
+        mixed_pass<true, RSET, T>(ca_b, p, m, ca.tw, ld_c, st_c);
+        flip();
+      }
+      mixed_pass<true, RSET, T>(ca_b, npc - 1, m, ca.tw, ld_c, st_w);
+    }
+    flip();
   }
 }
 
@@ -271,7 +217,8 @@ void* pick(int rset, bool dense) {
 }  // namespace
 
 size_t onecta_smem_bytes(int m, int ny, int row_ld, int col_ld) {
-  return (2 * (size_t)ny * row_ld + 2 * (size_t)m * col_ld + (size_t)m * ny) * sizeof(cplx<double>);
+  const size_t rows = (size_t)ny * row_ld, cols = (size_t)m * col_ld;
+  return (2 * (rows > cols ? rows : cols) + (size_t)m * ny) * sizeof(cplx<double>);
 }
 
 cudaError_t onecta_allow_smem(size_t bytes) {

@@ -1,6 +1,7 @@
 // Host side of the C ABI declared in include/pfc_b200.h: plan construction
 // (factorisation, twiddles, FP64 ETD1 coefficients, launch shapes), buffer
 // ownership and the launch sequences of each entry point.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -68,8 +69,7 @@ bool factorize(int n, bool fp32, std::vector<int>& radices) {
   return n == 1 && (int)radices.size() <= kMaxPass;
 }
 
-constexpr int kBlockMax = 256;  // default launch bound of the generic kernels
-constexpr int pfc_block_max = kBlockMax;
+constexpr int kBlockMax = 256;  // threads per CTA of the two-buffer kernels
 constexpr int kMaxElemsF = PFC_MAXE_F, kMaxElemsD = PFC_MAXE_D;  // as MaxElems in pfc_fft.cuh
 
 // must match MaxBfly in pfc_fft.cuh
@@ -85,6 +85,23 @@ bool all_pow2(const std::vector<int>& radices) {
   return true;
 }
 
+// Radices of the two-buffer engine, in descending order: the power-of-two part in as few
+// passes as radix 16 (FP32; FP64: 8, which bounds the registers of a butterfly) allows, split
+// evenly (16 = 4 x 4 in FP64, 32 = 8 x 4), then the odd primes.
+std::vector<int> mixed_radices(int n, bool fp32) {
+  std::vector<int> out;
+  int p2 = 0;
+  while (n % 2 == 0) { n /= 2; ++p2; }
+  const int cap = fp32 ? 4 : 3, np = (p2 + cap - 1) / cap;
+  for (int i = 0; i < np; ++i) out.push_back(1 << (p2 / np + (i < p2 % np ? 1 : 0)));
+  for (int r : {3, 5, 7, 11, 13})
+    while (n % r == 0) { out.push_back(r); n /= r; }
+  std::sort(out.rbegin(), out.rend());
+  return out;
+}
+
+unsigned div_magic(int d) { return d == 1 ? 0u : (unsigned)((1ULL << 32) / (unsigned)d) + 1u; }
+
 // Appends the pass tables of an n-point transform to `tw` (complex, long double
 // accuracy rounded once) and fills `d`.
 void build_fft(int n, const std::vector<int>& radices, std::vector<long double>& tw, FftDesc& d) {
@@ -96,6 +113,9 @@ void build_fft(int n, const std::vector<int>& radices, std::vector<long double>&
     const int R = radices[p];
     d.radix[p] = R;
     d.ns[p] = ns;
+    d.nr[p] = n / R;
+    d.mag_nr[p] = div_magic(n / R);
+    d.mag_ns[p] = div_magic(ns);
     d.twoff[p] = (int)(tw.size() / 2);
     // [q - 1][k]: the lanes of a warp (consecutive k) read consecutive entries
     for (int q = 1; q < R; ++q)
@@ -117,7 +137,7 @@ void build_fft(int n, const std::vector<int>& radices, std::vector<long double>&
     }
     ns *= R;
   }
-  for (int p = d.npass; p < kMaxPass; ++p) { d.radix[p] = 0; d.ns[p] = 0; d.twoff[p] = 0; d.rootoff[p] = -1; }
+  for (int p = d.npass; p < kMaxPass; ++p) { d.radix[p] = d.ns[p] = d.nr[p] = d.twoff[p] = 0; d.rootoff[p] = -1; }
 }
 
 int threads_per_fft(const std::vector<int>& radices, int n, bool fp32) {
@@ -156,10 +176,13 @@ struct pfc_plan {
   int* status = nullptr;
   // transforms and launch shapes
   FftDesc rowfft{}, colfft{};
+  FftDesc rowfft_b{}, colfft_b{};   // two-buffer kernels: the same radices in reverse order
   int rt_off = 0;       // offset of the real-packing twiddles in tw
   int row_tpf = 0, rows = 0, row_ld = 0, row_grid = 0, row_rset = kRadixPow2;
   int col_tpf = 0, cols = 0, col_ld = 0, col_grid = 0, col_rset = kRadixPow2;
   size_t row_smem = 0, col_smem = 0;
+  int row_block = 0, col_block = 0, rows_log2 = 0;   // threads per CTA of the run-time kernels
+  int par_tpf = 0, par_cols = 0, par_grid = 0;       // launch shape of the Parseval and export passes
   int cur = 0;
   bool state_set = false;
   long long steps_since_set = 0;
@@ -195,7 +218,7 @@ struct pfc_plan {
   // small FP64 mixed-radix grids: whole steps in one CTA (pfc_onecta.cu), reading this
   // plan's buffers from a one-entry table per parity of cur
   bool onecta = false;
-  int oc_threads = 0, oc_rset = kRadixPow2, oc_tpf_r = 0, oc_tpf_c = 0, oc_sms = 0;
+  int oc_threads = 0, oc_rset = kRadixPow2, oc_sms = 0;
   size_t oc_smem = 0;
   pfc::BatchBufs* oc_table[2] = {nullptr, nullptr};
 };
@@ -251,7 +274,8 @@ template <class T>
 RowArgs<T> row_args(const pfc_plan* h) {
   RowArgs<T> a{};
   a.nx = h->nx; a.ny = h->ny; a.m = h->m; a.rows = h->rows; a.tpf = h->row_tpf; a.ld = h->row_ld;
-  a.fft = h->rowfft;
+  a.rows_log2 = h->rows_log2;
+  a.fft = h->rowfft; a.fft_b = h->rowfft_b;
   a.tw = reinterpret_cast<const cplx<T>*>(h->tw);
   a.rtw = reinterpret_cast<const cplx<T>*>(h->tw) + h->rt_off;
   a.scal = h->scal;
@@ -268,7 +292,7 @@ ColArgs<T> col_args(const pfc_plan* h) {
   ColArgs<T> a{};
   a.nx = h->nx; a.ny = h->ny; a.m = h->m; a.cols = h->cols; a.tpf = h->col_tpf; a.ld = h->col_ld;
   a.nyh = h->nyh;
-  a.fft = h->colfft;
+  a.fft = h->colfft; a.fft_b = h->colfft_b;
   a.tw = reinterpret_cast<const cplx<T>*>(h->tw);
   a.coef = static_cast<const cplx<T>*>(h->coef);
   a.coef64 = static_cast<const cplx<double>*>(h->coef64);
@@ -293,17 +317,28 @@ template <class T, int MODE>
 int launch_row(pfc_plan* h, const RowArgs<T>& a, cudaStream_t s, int count = 1) {
   void* fn = pick_row<T, MODE>(h->prob.model, h->row_rset);
   void* args[] = {(void*)&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3(h->row_grid, count), dim3(h->rows * h->row_tpf), args, h->row_smem, s);
+  cudaError_t e = cudaLaunchKernel(fn, dim3(h->row_grid, count), dim3(h->row_block), args, h->row_smem, s);
   ++h->launches;
   if (e != cudaSuccess) return fail(PFC_E_CUDA, "row kernel launch failed: %s", cudaGetErrorString(e));
   return PFC_OK;
 }
 
 template <class T, int MODE>
-int launch_col(pfc_plan* h, const ColArgs<T>& a, cudaStream_t s, int count = 1) {
+int launch_col(pfc_plan* h, const ColArgs<T>& args_in, cudaStream_t s, int count = 1) {
   void* fn = pick_col<T, MODE>(h->col_rset);
+  ColArgs<T> a = args_in;
   void* args[] = {(void*)&a};
-  cudaError_t e = cudaLaunchKernel(fn, dim3(h->col_grid, count), dim3(h->cols * h->col_tpf), args, h->col_smem, s);
+  dim3 grid(h->col_grid, count), block(h->col_block);
+  size_t smem = h->col_smem;
+  if (MODE == kColParseval || MODE == kColExport) {
+    // no transform: threads along the columns, several short columns per CTA
+    a.cols = h->par_cols;
+    a.tpf = h->par_tpf;
+    grid.x = h->par_grid;
+    block.x = h->par_cols * h->par_tpf;
+    smem = 0;
+  }
+  cudaError_t e = cudaLaunchKernel(fn, grid, block, args, smem, s);
   ++h->launches;
   if (e != cudaSuccess) return fail(PFC_E_CUDA, "column kernel launch failed: %s", cudaGetErrorString(e));
   return PFC_OK;
@@ -331,8 +366,6 @@ int set_smem_attrs(pfc_plan* h) {
   PFC_ATTR((pick_col<T, kColStep>(cr)), h->col_smem);
   PFC_ATTR((pick_col<T, kColInit>(cr)), h->col_smem);
   PFC_ATTR((pick_col<T, kColCombine>(cr)), h->col_smem);
-  PFC_ATTR((pick_col<T, kColParseval>(cr)), h->col_smem);
-  PFC_ATTR((pick_col<T, kColExport>(cr)), h->col_smem);
 #undef PFC_ATTR
   return PFC_OK;
 }
@@ -811,25 +844,26 @@ int onecta_rset(int a, int b) {
 // Largest butterfly count of a pass of d: threads per transform for one butterfly each.
 int max_butterflies(const FftDesc& d) {
   int r = 1;
-  for (int p = 0; p < d.npass; ++p) r = std::max(r, d.n / d.radix[p]);
+  for (int p = 0; p < d.npass; ++p) r = std::max(r, d.nr[p]);
   return r;
 }
 
-// Chooses the one-CTA path for FP64 mixed-radix plans whose grid fits one CTA: every row
-// (and every column) transform at once within kOneCtaMaxThreads threads, up to one
-// butterfly per thread and pass, and the buffers within kOneCtaMaxSmem of shared memory.
-// PFC_FLAG_NO_ONE_CTA keeps the two-kernel step.
+// Chooses the one-CTA path for small FP64 mixed-radix plans. PFC_FLAG_NO_ONE_CTA keeps the
+// two-kernel step.
 int setup_onecta(pfc_plan* h) {
   h->onecta = false;
   if (h->fp32 || h->fast || (h->prob.flags & PFC_FLAG_NO_ONE_CTA)) return PFC_OK;
   const int rset = onecta_rset(h->row_rset, h->col_rset);
   if (rset < 0 || !onecta_supported(rset)) return PFC_OK;
-  const int tpf_r = std::min(max_butterflies(h->rowfft), std::max(1, kOneCtaMaxThreads / h->ny));
-  const int tpf_c = std::min(max_butterflies(h->colfft), std::max(1, kOneCtaMaxThreads / h->m));
-  const int need = std::max(h->ny * tpf_r, h->m * tpf_c);
-  const int threads = (need + 31) / 32 * 32;
+  // one thread per butterfly of the widest pass, at most a block
+  const int items = std::max(h->ny * max_butterflies(h->rowfft), h->m * max_butterflies(h->colfft));
+  const int threads = std::min((items + 31) / 32 * 32, kOneCtaMaxThreads);
   const size_t smem = onecta_smem_bytes(h->m, h->ny, h->row_ld, h->col_ld);
-  if (threads > kOneCtaMaxThreads || smem > kOneCtaMaxSmem) return PFC_OK;
+  // grids whose rows and columns, each in two buffers, and state take up to kOneCtaMaxSmem (the
+  // kernel itself holds the larger of rows and columns): beyond that one CTA's threads
+  // take longer than the launches it saves
+  const size_t footprint = (2 * ((size_t)h->ny * h->row_ld + (size_t)h->m * h->col_ld) + h->nspec) * sizeof(double2);
+  if (h->ny > kOneCtaMaxThreads || h->m > kOneCtaMaxThreads || footprint > kOneCtaMaxSmem) return PFC_OK;
   if (smem > 48 * 1024) {
     cudaError_t e = onecta_allow_smem(kOneCtaMaxSmem);
     if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
@@ -844,8 +878,6 @@ int setup_onecta(pfc_plan* h) {
   }
   h->onecta = true;
   h->oc_threads = threads;
-  h->oc_tpf_r = tpf_r;
-  h->oc_tpf_c = tpf_c;
   cudaDeviceGetAttribute(&h->oc_sms, cudaDevAttrMultiProcessorCount, h->device);
   h->oc_rset = rset;
   h->oc_smem = smem;
@@ -856,8 +888,6 @@ int setup_onecta(pfc_plan* h) {
 int launch_onecta(pfc_plan* h, cudaStream_t s, const BatchBufs* table, int count, long long nsteps) {
   RowArgs<double> ra = row_args<double>(h);
   ColArgs<double> ca = col_args<double>(h);
-  ra.tpf = h->oc_tpf_r;
-  ca.tpf = h->oc_tpf_c;
   // more plans than SMs: the build that fits two CTAs per SM
   const bool dense = count > h->oc_sms;
   cudaError_t e = launch_onecta_step(ra, ca, table, count, nsteps, h->prob.model, h->oc_rset, dense,
@@ -1045,6 +1075,9 @@ int do_step_timed(pfc_plan* h, long long nsteps, double* ms_row, double* ms_col,
   return rc;
 }
 
+// Threads of the final merge of n partials (one per partial up to a block).
+int merge_threads(int n) { return n <= 32 ? 32 : n <= 256 ? 256 : 1024; }
+
 template <class T>
 int do_materialize(pfc_plan* h, const void* spec, const double* add, double* out, bool correct_mean,
                    cudaStream_t s) {
@@ -1057,7 +1090,7 @@ int do_materialize(pfc_plan* h, const void* spec, const double* add, double* out
   if (rc) return rc;
   if (correct_mean) {
     const size_t sites = (size_t)h->nx * h->ny;
-    finalize_mean_kernel<<<1, 32, 0, s>>>(h->partials, h->row_grid, 1.0 / (double)sites, h->scal);
+    finalize_mean_kernel<<<1, merge_threads(h->row_grid), 0, s>>>(h->partials, h->row_grid, 1.0 / (double)sites, h->scal);
     ++h->launches;
     PFC_LAUNCHED();
     shift_kernel<<<1024, 256, 0, s>>>(out, sites, h->scal + kScalCorr);
@@ -1070,6 +1103,17 @@ int do_materialize(pfc_plan* h, const void* spec, const double* add, double* out
 template <class T>
 int do_get_state(pfc_plan* h, double* out, cudaStream_t s) {
   return do_materialize<T>(h, h->W, h->scal + (h->fp32 ? kScalMean : kScalZero), out, h->fp32, s);
+}
+
+BatchReduce reduce_params(const pfc_plan* h) {
+  BatchReduce b{};
+  const double dx = h->prob.lx / h->nx, dy = h->prob.ly / h->ny;
+  b.epsilon = h->prob.epsilon; b.beta = h->prob.beta; b.q0 = h->prob.q0;
+  b.fx = 1.0 / (h->nx * dx);
+  b.fy = 1.0 / (h->ny * dy);
+  b.lmu0 = h->lmu0; b.lf0 = h->lf0;
+  b.status = h->status;
+  return b;
 }
 
 template <class T>
@@ -1087,9 +1131,10 @@ int do_reduce(pfc_plan* h, double* out3, cudaStream_t s) {
   ca.partials = colp;
   rc = launch_col<T, kColParseval>(h, ca, s);
   if (rc) return rc;
-  const double sites = (double)h->nx * (double)h->ny;
-  finalize_reduce_kernel<<<1, 32, 0, s>>>(rowp, h->row_grid, colp, h->col_grid, h->scal, 1.0 / sites, h->lmu0,
-                                          h->lf0, h->fp32 ? 1 : 0, out3, h->status);
+  const BatchReduce br = reduce_params(h);
+  finalize_reduce_kernel<<<1, merge_threads(std::max(h->row_grid, h->par_grid)), 0, s>>>(
+      rowp, h->row_grid, colp, h->par_grid, 0, h->scal, br, nullptr, nullptr, nullptr,
+      1.0 / ((double)h->nx * (double)h->ny), h->fp32 ? 1 : 0, out3);
   ++h->launches;
   PFC_LAUNCHED();
   return PFC_OK;
@@ -1206,12 +1251,6 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   };
   h->row_rset = rset_of(rrow);
   h->col_rset = rset_of(rcol);
-  if (h->fp32 && (long long)p->nx * p->ny >= kDenseMinSites) {
-    for (int* r : {&h->row_rset, &h->col_rset}) {
-      if (*r == kRadixAll) *r = kRadixAllDense;
-      else if (*r == kRadixSmall) *r = kRadixSmallDense;
-    }
-  }
   h->elt = h->fp32 ? sizeof(float2) : sizeof(double2);
   cudaGetDevice(&h->device);
 
@@ -1219,8 +1258,20 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
 
   // ---- twiddles: row passes, column passes, real-packing table
   std::vector<long double> tw;
-  build_fft(m, rrow, tw, h->rowfft);
-  build_fft(p->ny, rcol, tw, h->colfft);
+  // two buffers of one padded transform fit an SM's shared memory: the two-buffer kernels,
+  // both radix orders; longer transforms: the one-buffer kernels
+  auto padded = [](int n) { const int ld = generic_pad(n - 1) + 2; return ld % 2 ? ld : ld + 1; };
+  const bool row_two = 2 * (size_t)padded(m) * h->elt <= kMixedSmem;
+  const bool col_two = 2 * (size_t)padded(p->ny) * h->elt <= kMixedSmem;
+  auto plan_fft = [&](int n, bool two, const std::vector<int>& one, FftDesc& d, FftDesc& db) {
+    if (!two) return build_fft(n, one, tw, d);
+    std::vector<int> r = mixed_radices(n, h->fp32);
+    build_fft(n, r, tw, d);
+    std::reverse(r.begin(), r.end());
+    build_fft(n, r, tw, db);
+  };
+  plan_fft(m, row_two, rrow, h->rowfft, h->rowfft_b);
+  plan_fft(p->ny, col_two, rcol, h->colfft, h->colfft_b);
   h->rt_off = (int)(tw.size() / 2);
   {
     const long double twopi = 6.283185307179586476925286766559L;
@@ -1246,53 +1297,63 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   int n_sm = 0;
   cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device);
   const int min_ctas = 2 * std::max(n_sm, 1);
+  // threads that one transform's widest pass can use, and the lengths the kernels take: up to
+  // 256 such threads, 1024 for radices up to 7
+  auto accept = [&](const char* what, int n, const std::vector<int>& one, int& tpf, int& rset, bool two) {
+    tpf = threads_per_fft(one, n, h->fp32);
+    const bool big = tpf > kBlockMax && rset != kRadixAll && tpf <= 1024;
+    if (tpf > kBlockMax && !big)
+      return fail(PFC_E_ARG, "pfc_plan_create: %s transform of %d points needs %d threads", what, n, tpf);
+    if ((size_t)padded(n) * cbytes > (size_t)budget)
+      return fail(PFC_E_ARG, "pfc_plan_create: %s transform of %d points does not fit", what, n);
+    if (!two) rset = rset == kRadixPow2 ? kRadixPow2Big : kRadixSmallBig;
+    return (int)PFC_OK;
+  };
+  auto block_of = [](const FftDesc& d, int count) {   // one thread per butterfly of the widest pass, at most 256
+    int items = 1;
+    for (int p = 0; p < d.npass; ++p) items = std::max(items, count * d.nr[p]);
+    return std::min(256, (items + 31) / 32 * 32);
+  };
   {
-    h->row_tpf = threads_per_fft(rrow, m, h->fp32);
-    // padded row (generic_pad) plus one, odd, so that the transposing tile accesses of
-    // consecutive rows start on different banks
-    h->row_ld = generic_pad(m - 1) + 2;
-    if (h->row_ld % 2 == 0) ++h->row_ld;
-    if (h->row_tpf > kBlockMax && h->row_rset == kRadixPow2 && h->row_tpf <= 1024) h->row_rset = kRadixPow2Big;
-    if (h->row_tpf > kBlockMax && (h->row_rset == kRadixSmall || h->row_rset == kRadixSmallDense) &&
-        h->row_tpf <= 1024)
-      h->row_rset = kRadixSmallBig;
-    const int kBlockMax = (h->row_rset == kRadixPow2Big || h->row_rset == kRadixSmallBig) ? 1024 : pfc_block_max;
-    if (h->row_tpf > kBlockMax)
-      return cleanup_fail(fail(PFC_E_ARG, "pfc_plan_create: row transform of %d points needs %d threads", m, h->row_tpf));
+    if (int rc = accept("row", m, rrow, h->row_tpf, h->row_rset, row_two)) return cleanup_fail(rc);
+    h->row_ld = padded(m);   // odd, so that the transposing tile accesses of consecutive rows start on different banks
     const int rows_min = std::max(1, 32 / h->row_tpf);       // whole warps
-    const int rows_cap = std::max(rows_min, kBlockMax / h->row_tpf);
-    const int coalesce = std::max(1, 64 / cbytes);           // >= 64 B per kx run
-    int rows = std::max(rows_min, std::min(coalesce, rows_cap));
-    while (2 * rows <= rows_cap && (size_t)(2 * rows) * h->row_ld * cbytes <= (size_t)budget / 2 && rows < p->ny)
-      rows *= 2;
-    while ((size_t)rows * h->row_ld * cbytes > (size_t)budget && rows > std::max(1, 32 / h->row_tpf)) rows /= 2;
-    while (rows > rows_min && (p->ny + rows - 1) / rows < min_ctas) rows /= 2;
-    if ((size_t)rows * h->row_ld * cbytes > (size_t)budget || rows * h->row_tpf > kBlockMax)
-      return cleanup_fail(fail(PFC_E_ARG, "pfc_plan_create: row transform of %d points does not fit", m));
+    int rows = rows_min;
+    if (row_two) {
+      // >= 64 B per kx run where two CTAs fit an SM, at least two CTAs per SM where the grid allows it
+      rows = std::max(rows_min, std::max(1, 64 / cbytes));
+      while (rows > rows_min && 2 * (size_t)rows * h->row_ld * cbytes > kMixedSmem / 2) rows /= 2;
+      while (rows > rows_min && (p->ny + rows - 1) / rows < min_ctas) rows /= 2;
+      h->row_block = block_of(h->rowfft, rows);
+    } else {
+      h->row_block = rows * h->row_tpf;
+    }
     h->rows = rows;
+    h->rows_log2 = ilog2_exact(rows);
     h->row_grid = (p->ny + rows - 1) / rows;
-    h->row_smem = (size_t)rows * h->row_ld * cbytes;
+    h->row_smem = (row_two ? 2 : 1) * (size_t)rows * h->row_ld * cbytes;
   }
   {
-    h->col_tpf = threads_per_fft(rcol, p->ny, h->fp32);
-    h->col_ld = generic_pad(p->ny - 1) + 2;   // padded column plus one
-    if (h->col_ld % 2 == 0) ++h->col_ld;
-    if (h->col_tpf > kBlockMax && h->col_rset == kRadixPow2 && h->col_tpf <= 1024) h->col_rset = kRadixPow2Big;
-    if (h->col_tpf > kBlockMax && (h->col_rset == kRadixSmall || h->col_rset == kRadixSmallDense) &&
-        h->col_tpf <= 1024)
-      h->col_rset = kRadixSmallBig;
-    const int kBlockMax = (h->col_rset == kRadixPow2Big || h->col_rset == kRadixSmallBig) ? 1024 : pfc_block_max;
-    if (h->col_tpf > kBlockMax)
-      return cleanup_fail(fail(PFC_E_ARG, "pfc_plan_create: column transform of %d points needs %d threads", p->ny, h->col_tpf));
-    int cols = std::max(1, 32 / h->col_tpf);
-    while (2 * cols * h->col_tpf <= kBlockMax && (size_t)(2 * cols) * h->col_ld * cbytes <= (size_t)budget / 2 && cols < m)
-      cols *= 2;
-    while (cols > std::max(1, 32 / h->col_tpf) && (m + cols - 1) / cols < min_ctas) cols /= 2;
-    if ((size_t)cols * h->col_ld * cbytes > (size_t)budget || cols * h->col_tpf > kBlockMax)
-      return cleanup_fail(fail(PFC_E_ARG, "pfc_plan_create: column transform of %d points does not fit", p->ny));
+    if (int rc = accept("column", p->ny, rcol, h->col_tpf, h->col_rset, col_two)) return cleanup_fail(rc);
+    h->col_ld = padded(p->ny);
+    const int cols_min = std::max(1, 32 / h->col_tpf);
+    int cols = cols_min;
+    if (col_two) {
+      while (2 * cols * h->col_tpf <= kBlockMax && 2 * (size_t)(2 * cols) * h->col_ld * cbytes <= kMixedSmem / 2 && cols < m)
+        cols *= 2;
+      while (cols > cols_min && (m + cols - 1) / cols < min_ctas) cols /= 2;
+      h->col_block = block_of(h->colfft, cols);
+    } else {
+      h->col_block = cols * h->col_tpf;
+    }
     h->cols = cols;
     h->col_grid = (m + cols - 1) / cols;
-    h->col_smem = (size_t)cols * h->col_ld * cbytes;
+    h->col_smem = (col_two ? 2 : 1) * (size_t)cols * h->col_ld * cbytes;
+    h->par_tpf = 32;
+    while (h->par_tpf < 256 && h->par_tpf * 8 < p->ny) h->par_tpf *= 2;
+    h->par_cols = std::min(256 / h->par_tpf, m);
+    while (h->par_cols > 1 && (m + h->par_cols - 1) / h->par_cols < min_ctas) h->par_cols /= 2;
+    h->par_grid = (m + h->par_cols - 1) / h->par_cols;
   }
 
   // ---- FP64 ETD1 coefficients (kernels.py:55-71) and the update factor Gamma*lap
@@ -1341,7 +1402,7 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   if (e == cudaSuccess) e = cudaMalloc(&h->V, specb);
   if (e == cudaSuccess) e = cudaMalloc(&h->coef, ncoef * h->elt);
   if (e == cudaSuccess) e = cudaMalloc(&h->tw, tw.size() / 2 * h->elt);
-  h->npartials = 6 * (size_t)h->row_grid + 2 * (size_t)h->col_grid + 2 * 1024;
+  h->npartials = 6 * (size_t)h->row_grid + 2 * (size_t)h->par_grid + 2 * 1024;
   if (e == cudaSuccess) e = cudaMalloc(&h->partials, h->npartials * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->scal, kScalCount * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->status, sizeof(int));

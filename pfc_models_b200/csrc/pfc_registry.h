@@ -9,22 +9,14 @@
 
 namespace pfc {
 
-// Radix-set code of the generic kernels built for 1024-thread blocks, used when one
-// transform needs more than 256 threads (>= 8192 points in FP32); kRadixPow2 and
-// kRadixAll (pfc_fft.cuh) select the 256-thread kernels.
+// Radix-set codes of the run-time kernels: kRadixPow2, kRadixSmall and kRadixAll
+// (pfc_fft.cuh) select the two-buffer kernels (pfc_mixed.cuh); the codes below the one-buffer
+// kernels (pfc_kernels.cuh, 1024-thread blocks) for transforms whose two buffers exceed
+// kMixedSmem of shared memory (FP64 8192 points), with power-of-two radices or with the
+// radices up to 7. (Lengths with a factor 11 or 13 always fit two buffers.)
 constexpr int kRadixPow2Big = 2;
-// The all-radix step kernels (row and column) built for two CTAs per SM (at most 128
-// registers, with some spills) instead of one: faster for large FP32 grids, slower for
-// small grids and in FP64 (measured on B200). Modes other than the step use kRadixAll.
-constexpr int kRadixAllDense = 3;
-// Grids with prime factors 2, 3, 5, 7 only: the smaller radix set (kRadixSmall), and its
-// two-CTA step build as above.
-constexpr int kRadixSmallDense = 5;
-// The small-radix generic kernels built for 1024-thread blocks: transforms whose radix-5 or
-// radix-7 pass has more than 256 butterflies (2560 = 5 x 512, 3584 = 7 x 512, 5120 points);
-// they hold one butterfly of such a pass per thread, so the block grows with the length.
 constexpr int kRadixSmallBig = 6;
-constexpr long long kDenseMinSites = 1LL << 20;
+constexpr size_t kMixedSmem = 200 * 1024;
 
 // log2 sizes of the power-of-two step kernels: row transforms of M = nx/2 points,
 // column transforms of ny points
