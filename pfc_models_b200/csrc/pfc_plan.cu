@@ -221,6 +221,9 @@ struct pfc_plan {
   int oc_threads = 0, oc_rset = kRadixPow2, oc_sms = 0;
   size_t oc_smem = 0;
   pfc::BatchBufs* oc_table[2] = {nullptr, nullptr};
+  bool dense = false;          // its transforms as matrix products
+  pfc::DenseArgs dense_args{};
+  int dense_row = 0, dense_col = 0;   // their tables' offsets in tw
 };
 
 // A batch of plans stepped in lockstep: plans with the same step kernels, sizes and
@@ -876,6 +879,21 @@ int setup_onecta(pfc_plan* h) {
     if (e == cudaSuccess) e = cudaMemcpy(h->oc_table[p], &b, sizeof(BatchBufs), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA table: %s", cudaGetErrorString(e));
   }
+  if (h->dense) {
+    DenseArgs& d = h->dense_args;
+    const size_t bytes = dense_shape(h->m, h->ny, d);
+    const double2* tw = reinterpret_cast<const double2*>(h->tw);
+    const RowArgs<double> ra = row_args<double>(h);
+    d.row_tab = tw + h->dense_row;
+    d.col_tab = tw + h->dense_col;
+    d.g = ra.g; d.min_phi = ra.min_phi; d.min_log = ra.min_log; d.clamp = ra.clamp;
+    d.scale = col_args<double>(h).scale;
+    cudaError_t e = dense_allow_smem(kOneCtaMaxSmem);
+    if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
+    h->oc_smem = bytes;
+    h->onecta = true;
+    return PFC_OK;
+  }
   h->onecta = true;
   h->oc_threads = threads;
   cudaDeviceGetAttribute(&h->oc_sms, cudaDevAttrMultiProcessorCount, h->device);
@@ -886,6 +904,12 @@ int setup_onecta(pfc_plan* h) {
 
 // `nsteps` steps of `count` plans of one class (table: their buffers at the current parity).
 int launch_onecta(pfc_plan* h, cudaStream_t s, const BatchBufs* table, int count, long long nsteps) {
+  if (h->dense) {
+    cudaError_t e = launch_dense_step(h->dense_args, table, count, nsteps, h->prob.model, h->oc_smem, s);
+    ++h->launches;
+    if (e != cudaSuccess) return fail(PFC_E_CUDA, "one-CTA step launch failed: %s", cudaGetErrorString(e));
+    return PFC_OK;
+  }
   RowArgs<double> ra = row_args<double>(h);
   ColArgs<double> ca = col_args<double>(h);
   // more plans than SMs: the build that fits two CTAs per SM
@@ -1284,6 +1308,17 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   {
     const int rc = h->fp32 ? setup_fast<float>(h, tw) : setup_fast<double>(h, tw);
     if (rc) return cleanup_fail(rc);
+  }
+
+  if (!h->fp32 && !h->fast && !(p->flags & (PFC_FLAG_NO_ONE_CTA | PFC_FLAG_EXTV))) {
+    h->dense = dense_shape(m, p->ny, h->dense_args) <= kOneCtaMaxSmem &&
+               dense_products(h->dense_args) <= kDenseMaxProducts;
+    if (h->dense) {
+      h->dense_row = (int)(tw.size() / 2);
+      dense_table(p->nx, tw);
+      h->dense_col = (int)(tw.size() / 2);
+      dense_table(p->ny, tw);
+    }
   }
 
   // ---- launch shapes

@@ -108,6 +108,29 @@ cudaError_t launch_onecta_step(const RowArgs<double>& ra, const ColArgs<double>&
                                int count, long long nsteps, int model, int rset, bool dense, int threads,
                                size_t smem, cudaStream_t stream);
 
+// The same step with dense transforms on the FP64 tensor cores (onecta_dense_kernel).
+struct DenseArgs {
+  int m, ny, nyh;                  // half row length, column length, coefficients a column
+  int tr, kr, tc, kc;              // 8-wide output tiles and 4-deep steps of the row and column matrices
+  int ys, ks, cpad;                // strides of the [.][y] and [.][ky] arrays, real columns padded to 8
+  int size_a, size_b;              // doubles of the two work areas
+  const double2 *row_tab, *col_tab;
+  double g, min_phi, min_log, scale;
+  int clamp;
+};
+size_t dense_shape(int m, int ny, DenseArgs& a);           // fills the sizes; bytes of shared memory
+int dense_products(const DenseArgs& a);                    // m8n8k4 products of a step
+// Plans of up to this many products a step take the dense transforms. Their cost grows with
+// the square of the sides. B200, us a step, one cell / 296 cells in one batch, dense against
+// FFT passes: 28 x 24 (224 products) 2.0 / 2.8 against 6.0 / 6.3, 48 x 20 (512) 3.7 / 4.8
+// against 5.5 / 6.2, 30 x 50 (672) 4.2 / 5.9 against 6.4 / 7.6, 32 x 56 (932) 5.4 / 7.9
+// against 6.6 / 7.8 and for the log model 7.4 / 10.6 against 8.0 / 9.6.
+constexpr int kDenseMaxProducts = 800;
+void dense_table(int n, std::vector<long double>& tw);     // appends the (w cos, w sin) fragments of length n
+cudaError_t dense_allow_smem(size_t bytes);
+cudaError_t launch_dense_step(const DenseArgs& args, const BatchBufs* table, int count, long long nsteps, int model,
+                              size_t smem, cudaStream_t stream);
+
 // Log PFC with an external potential (pfc_extv.cu): the state of the M shift, kept in
 // device memory, and the arguments of the coefficient rebuild.
 struct ExtvState {

@@ -128,3 +128,35 @@ def test_batch_mixing_one_cta_and_two_kernel_classes_equals_plans_alone():
     for i, (s, t) in enumerate(zip(sims, alone)):
         assert np.array_equal(s.plan.get_state().cpu().numpy(), t.plan.get_state().cpu().numpy()), i
     b.close()
+
+
+# dense transforms: odd and even sides, sides of one tile and just past one, the shortest; the
+# last two sizes lie on either side of the product count up to which plans take them
+DENSE_GRIDS = [(4, 2), (4, 3), (6, 5), (10, 7), (14, 9), (16, 15), (18, 16), (30, 22), (14, 33), (28, 24), (30, 50),
+               (32, 56)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", DENSE_GRIDS)
+@pytest.mark.parametrize("model", ["std", "log"])
+def test_one_cta_transforms_against_oracle(model, nx, ny):
+    """Matrix products round each output like a sum of n / 2 terms: a few ulp, as the FFT
+    passes; 25 steps within 1e-12 relative L2 of the oracle, in launches of odd and even
+    length, mu (from V and the previous state, which the last step leaves) included."""
+    from oracle import pfc_oracle as orc
+    sim = _sim(model, nx, ny, True)
+    assert sim.plan.path() == "one_cta"
+    m, g = sim.Model, sim.Geometry
+    o = orc.OracleSim(model, orc.Params(Gamma=m.Gamma, beta=m.beta, q0=m.q0, epsilon=m.epsilon, g=m.g, dt=m.dt),
+                      orc.build_geometry(nx, ny, g.Lx, g.Ly))
+    o.set_field(sim.plan.get_state().cpu().numpy())
+    for n in (1, 14, 10):
+        sim.TimeSteps(n)
+        for _ in range(n):
+            mu = o.mu()
+            o.step()
+        got = sim.plan.get_state().cpu().numpy()
+        assert np.linalg.norm(got - o.n) <= 1e-12 * np.linalg.norm(o.n), n
+        lmu = float(np.max(np.abs(o.lin_mu)))
+        assert np.linalg.norm(sim.mu.get() - mu) <= 1e-12 * (np.linalg.norm(mu) + lmu * np.linalg.norm(o.n)), n
+        assert sim.CalculateFreeEnergy() == pytest.approx(o.free_energy(), rel=1e-12, abs=1e-13)
