@@ -73,6 +73,7 @@ SIGNATURES = {
     "pfc_field_mean_noalloc": (ctypes.c_int, [_vp, _i64, _vp, _vp]),
     "pfc_batch_create": (ctypes.c_int, [ctypes.POINTER(_vp), _i32, ctypes.POINTER(_vp)]),
     "pfc_batch_step": (ctypes.c_int, [_vp, _i64, _vp]),
+    "pfc_batch_reduce": (ctypes.c_int, [_vp, _vp, _vp]),
     "pfc_batch_destroy": (ctypes.c_int, [_vp]),
     "pfc_batch_launch_count": (_i64, [_vp]),
     "pfc_batch_classes": (ctypes.c_int, [_vp]),

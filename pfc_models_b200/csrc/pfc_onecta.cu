@@ -482,19 +482,18 @@ int dense_products(const DenseArgs& a) {
   return 4 * ((a.ny + 7) / 8 * a.tr * a.kr + a.cpad / 8 * a.tc * a.kc);
 }
 
-void dense_table(int n, std::vector<long double>& tw) {
+void dense_table(int n, const std::vector<long double>& root, std::vector<long double>& tw) {
   const int h = n / 2, tiles = h / 8 + 1, steps = h / 4 + 1;
-  const long double twopi = 6.283185307179586476925286766559L;
   for (int t = 0; t < tiles; ++t)
     for (int q = 0; q < steps; ++q)
       for (int lane = 0; lane < 32; ++lane) {
         const int out = 8 * t + lane / 4, in = 4 * q + lane % 4;
         long double c = 0, s = 0;
         if (out <= h && in <= h) {
-          const long long num = (long long)out * in % n;
-          const long double w = (in == 0 || 2 * in == n) ? 0.5L : 1.0L, ang = twopi * (long double)num / (long double)n;
-          c = w * cosl(ang);
-          s = (2 * num) % n == 0 ? 0.0L : w * sinl(ang);
+          const int k = out * in % n;
+          const long double w = (in == 0 || 2 * in == n) ? 0.5L : 1.0L;
+          c = w * root[2 * k];
+          s = 2 * k % n == 0 ? 0.0L : -w * root[2 * k + 1];
         }
         tw.push_back(c);
         tw.push_back(s);

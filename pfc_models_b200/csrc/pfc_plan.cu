@@ -102,10 +102,27 @@ std::vector<int> mixed_radices(int n, bool fp32) {
 
 unsigned div_magic(int d) { return d == 1 ? 0u : (unsigned)((1ULL << 32) / (unsigned)d) + 1u; }
 
-// Appends the pass tables of an n-point transform to `tw` (complex, long double
-// accuracy rounded once) and fills `d`.
-void build_fft(int n, const std::vector<int>& radices, std::vector<long double>& tw, FftDesc& d) {
+// exp(-2 pi i k / n), k < n, in long double (each trigonometric value of a plan's tables is
+// evaluated once: a pass's angles are multiples of 2 pi / n)
+std::vector<long double> unit_roots(int n) {
   const long double twopi = 6.283185307179586476925286766559L;
+  std::vector<long double> r(2 * (size_t)n);
+  for (int k = 0; k < n; ++k) {
+    const long double ang = -twopi * (long double)k / (long double)n;
+    r[2 * k] = cosl(ang);
+    r[2 * k + 1] = sinl(ang);
+  }
+  return r;
+}
+
+// Appends the pass tables of an n-point transform to `tw` (complex, long double
+// accuracy rounded once) and fills `d`. root = unit_roots(n).
+void build_fft(int n, const std::vector<int>& radices, const std::vector<long double>& root,
+               std::vector<long double>& tw, FftDesc& d) {
+  auto push = [&](long long k) {
+    tw.push_back(root[2 * k]);
+    tw.push_back(root[2 * k + 1]);
+  };
   d.n = n;
   d.npass = (int)radices.size();
   int ns = 1;
@@ -119,19 +136,10 @@ void build_fft(int n, const std::vector<int>& radices, std::vector<long double>&
     d.twoff[p] = (int)(tw.size() / 2);
     // [q - 1][k]: the lanes of a warp (consecutive k) read consecutive entries
     for (int q = 1; q < R; ++q)
-      for (int k = 0; k < ns; ++k) {
-        const long long num = (long long)q * k % ((long long)ns * R);
-        const long double ang = -twopi * (long double)num / (long double)(ns * R);
-        tw.push_back(cosl(ang));
-        tw.push_back(sinl(ang));
-      }
+      for (int k = 0; k < ns; ++k) push((long long)q * k % ((long long)ns * R) * (n / (ns * R)));
     if (R >= 5) {
       d.rootoff[p] = (int)(tw.size() / 2);
-      for (int mm = 0; mm < R; ++mm) {
-        const long double ang = -twopi * (long double)mm / (long double)R;
-        tw.push_back(cosl(ang));
-        tw.push_back(sinl(ang));
-      }
+      for (int mm = 0; mm < R; ++mm) push((long long)mm * (n / R));
     } else {
       d.rootoff[p] = -1;
     }
@@ -231,9 +239,14 @@ struct pfc_plan {
 // gridDim.y = plans in the class.
 struct pfc_batch_class {
   std::vector<pfc_plan*> plans;
+  std::vector<int> rows;                          // their places in the caller's list
   pfc::BatchBufs* table[2] = {nullptr, nullptr};  // device tables, by parity of cur
   cudaStream_t stream = nullptr;                  // classes run concurrently (fork/join)
   cudaEvent_t done = nullptr;
+  // batched reductions: the plans' parameters, their rows of the output, their partials
+  pfc::BatchReduce* red = nullptr;
+  int* slot = nullptr;
+  double* partials = nullptr;
 };
 
 struct pfc_batch {
@@ -1164,6 +1177,49 @@ int do_reduce(pfc_plan* h, double* out3, cudaStream_t s) {
   return PFC_OK;
 }
 
+// Partials of one plan's reduction: 3 sums per row CTA, 1 per Parseval CTA.
+size_t reduce_partials(const pfc_plan* h) { return 6 * (size_t)h->row_grid + 2 * (size_t)h->par_grid; }
+
+// The reductions of every plan: per class one launch of each of the three kernels of
+// do_reduce, one grid row (or block) per plan, so that each plan's sums are formed as
+// do_reduce forms them. Plans of a class that were stepped apart (other parities) reduce
+// one by one.
+template <class T>
+int do_batch_reduce(pfc_batch* b, double* out, cudaStream_t s) {
+  for (auto& c : b->classes)
+    for (pfc_plan* h : c.plans)
+      if (!h->state_set) return fail(PFC_E_STATE, "pfc_batch_reduce: a plan has no state");
+  for (auto& c : b->classes) {
+    pfc_plan* h = c.plans[0];
+    const int n = (int)c.plans.size();
+    bool together = true;
+    for (pfc_plan* q : c.plans) together = together && q->cur == h->cur;
+    if (!together) {
+      for (int i = 0; i < n; ++i)
+        if (int rc = do_reduce<T>(c.plans[i], out + 3 * (size_t)c.rows[i], s)) return rc;
+      continue;
+    }
+    const BatchBufs* table = c.table[h->cur];
+    const int stride = (int)reduce_partials(h);
+    RowArgs<T> ra = row_args<T>(h);
+    ra.partials = c.partials;
+    ra.batch = table; ra.red = c.red; ra.partials_stride = stride;
+    int rc = launch_row<T, kRowReduce>(h, ra, s, n);
+    if (rc) return rc;
+    ColArgs<T> ca = col_args<T>(h);
+    double* colp = c.partials + 6 * (size_t)h->row_grid;
+    ca.partials = colp;
+    ca.batch = table; ca.red = c.red; ca.partials_stride = stride;
+    rc = launch_col<T, kColParseval>(h, ca, s, n);
+    if (rc) return rc;
+    finalize_reduce_kernel<<<n, merge_threads(std::max(h->row_grid, h->par_grid)), 0, s>>>(
+        c.partials, h->row_grid, colp, h->par_grid, stride, nullptr, BatchReduce{}, table, c.red, c.slot,
+        1.0 / ((double)h->nx * (double)h->ny), h->fp32 ? 1 : 0, out);
+    PFC_LAUNCHED();
+  }
+  return PFC_OK;
+}
+
 // Nonlinear row spectra V of the "previous" state, and the index of that state's n_hat.
 template <class T>
 int prepare_previous(pfc_plan* h, bool current, int* old_buf, cudaStream_t s) {
@@ -1288,11 +1344,12 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   const bool row_two = 2 * (size_t)padded(m) * h->elt <= kMixedSmem;
   const bool col_two = 2 * (size_t)padded(p->ny) * h->elt <= kMixedSmem;
   auto plan_fft = [&](int n, bool two, const std::vector<int>& one, FftDesc& d, FftDesc& db) {
-    if (!two) return build_fft(n, one, tw, d);
+    const std::vector<long double> root = unit_roots(n);
+    if (!two) return build_fft(n, one, root, tw, d);
     std::vector<int> r = mixed_radices(n, h->fp32);
-    build_fft(n, r, tw, d);
+    build_fft(n, r, root, tw, d);
     std::reverse(r.begin(), r.end());
-    build_fft(n, r, tw, db);
+    build_fft(n, r, root, tw, db);
   };
   plan_fft(m, row_two, rrow, h->rowfft, h->rowfft_b);
   plan_fft(p->ny, col_two, rcol, h->colfft, h->colfft_b);
@@ -1315,9 +1372,9 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
                dense_products(h->dense_args) <= kDenseMaxProducts;
     if (h->dense) {
       h->dense_row = (int)(tw.size() / 2);
-      dense_table(p->nx, tw);
+      dense_table(p->nx, unit_roots(p->nx), tw);
       h->dense_col = (int)(tw.size() / 2);
-      dense_table(p->ny, tw);
+      dense_table(p->ny, unit_roots(p->ny), tw);
     }
   }
 
@@ -1665,6 +1722,7 @@ int pfc_batch_create(pfc_plan* const* plans, int32_t count, pfc_batch** out) {
       cls = &b->classes.back();
     }
     cls->plans.push_back(h);
+    cls->rows.push_back(i);
   }
   cudaError_t es = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
   for (auto& c : b->classes) {
@@ -1699,8 +1757,28 @@ int pfc_batch_create(pfc_plan* const* plans, int32_t count, pfc_batch** out) {
       }
     }
   }
+  for (auto& c : b->classes) {
+    const size_t n = c.plans.size();
+    std::vector<BatchReduce> red(n);
+    for (size_t i = 0; i < n; ++i) red[i] = reduce_params(c.plans[i]);
+    cudaError_t e = cudaMalloc(&c.red, n * sizeof(BatchReduce));
+    if (e == cudaSuccess) e = cudaMalloc(&c.slot, n * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&c.partials, n * reduce_partials(c.plans[0]) * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemcpy(c.red, red.data(), n * sizeof(BatchReduce), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(c.slot, c.rows.data(), n * sizeof(int), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      pfc_batch_destroy(b);
+      return fail(PFC_E_CUDA, "pfc_batch_create: %s", cudaGetErrorString(e));
+    }
+  }
   *out = b;
   return PFC_OK;
+}
+
+int pfc_batch_reduce(pfc_batch* b, double* out, void* stream) {
+  if (!b || !out) return fail(PFC_E_ARG, "pfc_batch_reduce: null argument");
+  cudaStream_t s = (cudaStream_t)stream;
+  return b->fp32 ? do_batch_reduce<float>(b, out, s) : do_batch_reduce<double>(b, out, s);
 }
 
 int pfc_batch_step(pfc_batch* b, int64_t nsteps, void* stream) {
@@ -1716,7 +1794,7 @@ int pfc_batch_destroy(pfc_batch* b) {
   for (auto& g : b->graph)
     if (g) cudaGraphExecDestroy(g);
   for (auto& c : b->classes) {
-    for (auto& tb : c.table)
+    for (void* tb : {(void*)c.table[0], (void*)c.table[1], (void*)c.red, (void*)c.slot, (void*)c.partials})
       if (tb) cudaFree(tb);
     if (c.done) cudaEventDestroy(c.done);
     if (c.stream) cudaStreamDestroy(c.stream);

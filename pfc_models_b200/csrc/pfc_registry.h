@@ -126,7 +126,8 @@ int dense_products(const DenseArgs& a);                    // m8n8k4 products of
 // against 5.5 / 6.2, 30 x 50 (672) 4.2 / 5.9 against 6.4 / 7.6, 32 x 56 (932) 5.4 / 7.9
 // against 6.6 / 7.8 and for the log model 7.4 / 10.6 against 8.0 / 9.6.
 constexpr int kDenseMaxProducts = 800;
-void dense_table(int n, std::vector<long double>& tw);     // appends the (w cos, w sin) fragments of length n
+// appends the (w cos, w sin) fragments of length n; root = exp(-2 pi i k / n), k < n
+void dense_table(int n, const std::vector<long double>& root, std::vector<long double>& tw);
 cudaError_t dense_allow_smem(size_t bytes);
 cudaError_t launch_dense_step(const DenseArgs& args, const BatchBufs* table, int count, long long nsteps, int model,
                               size_t smem, cudaStream_t stream);

@@ -43,6 +43,13 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+def _advanced(t, dt, nsteps):
+    """t after `nsteps` additions of dt, rounded one by one as a TimeStep loop rounds them."""
+    a = np.full(nsteps + 1, dt, dtype=np.float64)
+    a[0] = t
+    return np.add.accumulate(a)[-1]
+
+
 class ModelParameters:
     """Parameter holder; ints and float64 scalars are stored as np.float64, lists and
     tuples as float64 arrays (models/stdpfc/simulation.py:40-58)."""
@@ -454,8 +461,7 @@ class Simulation:
         self._plan.step(nsteps)
         self._version += 1
         self._mu_current = False
-        for _ in range(nsteps):
-            self.State.t += self.Model.dt
+        self.State.t = _advanced(self.State.t, self.Model.dt, nsteps)
 
     # mirrors of the reference's batch hooks: after these, State.mu refers to the current field
     def _Batch1_CalcNonlinMu(self):
@@ -518,24 +524,31 @@ class Batch:
         if nsteps <= 0:
             return
         self._step_call(nsteps)
+        # members at the same time with the same dt share the sum (a loop over 252 members'
+        # 1000 steps took 12 ms, as long as the steps themselves on the device)
+        times = {}
         for s in self.items:
             if isinstance(s, Simulation):
                 s._version += 1
                 s._mu_current = False
-                for _ in range(nsteps):
-                    s.State.t += s.Model.dt
+                key = (s.State.t, s.Model.dt)
+                if key not in times:
+                    times[key] = _advanced(*key, nsteps)
+                s.State.t = times[key]
 
     def _step_call(self, nsteps):
         _lib.check(self.lib.pfc_batch_step(self.handle, nsteps, _stream_ptr(self.torch, self.device)))
 
     def reduce(self):
         """(F per site, mu per site, mean density) of every simulation as an (n, 3) FP64
-        array, with one device-to-host copy for the whole batch."""
+        array: three launches per class and one device-to-host copy for the whole batch."""
         t = self.torch
         out = t.empty((len(self.plans), 3), dtype=t.float64, device=self.device)
-        for i, p in enumerate(self.plans):
-            p.reduce(out[i])
+        self._reduce_call(out)
         return out.cpu().numpy()
+
+    def _reduce_call(self, out):
+        _lib.check(self.lib.pfc_batch_reduce(self.handle, _ptr(out), _stream_ptr(self.torch, self.device)))
 
     @property
     def classes(self):
@@ -580,6 +593,10 @@ class QueueBatch(Batch):
 
     def _step_call(self, nsteps):
         _lib.check(self.lib.pfc_queue_step(self.handle, nsteps, _stream_ptr(self.torch, self.device)))
+
+    def _reduce_call(self, out):
+        for i, p in enumerate(self.plans):
+            p.reduce(out[i])
 
     def status(self):
         """Status bits of the launches so far (synchronises): 0, or STATUS_TIMEOUT when a

@@ -230,3 +230,34 @@ def test_nonfinite_member_is_flagged_alone(precision):
         ref[i].TimeSteps(37)
         assert np.array_equal(_field(sims[i]), _field(ref[i])), i
     b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_batch_reduce_equals_each_plans_own(precision):
+    """One launch per class and kernel: bit for bit each plan's own reduction, in the caller's
+    order, for interleaved classes with parameters and boxes of their own, at odd and even step
+    counts and with members stepped apart (no common parity)."""
+    specs = [(128, 64, -0.3), (36, 20, -0.2), (128, 64, -0.25), (30, 22, -0.35), (36, 20, -0.4), (128, 64, -0.1)]
+    sims = []
+    for i, (nx, ny, eps) in enumerate(specs):
+        prm = stdpfc.BuildStdPFCModelParameters(Gamma=1.0, beta=1.0 + 0.1 * i, q0=1.0, epsilon=eps, g=0.0, dt=0.3)
+        s = stdpfc.BuildB200_Simulation(prm, stdpfc.Build2DGeometry(nx, ny, nx * (0.7 + 0.01 * i), ny * 0.8),
+                                        precision=precision)
+        s.State.n[...] = -0.3 + 0.05 * np.random.default_rng(i).uniform(-1, 1, (ny, nx))
+        sims.append(s)
+    b = Batch(sims)
+    for n in (0, 3, 1):
+        b.step(n)
+        assert [tuple(r) for r in b.reduce()] == [s.Reduce() for s in sims], n
+    sims[2].TimeStep()
+    assert [tuple(r) for r in b.reduce()] == [s.Reduce() for s in sims]
+    b.close()
+
+
+def test_time_advances_as_single_steps_round():
+    """State.t after a block equals a loop of additions bit for bit."""
+    from pfc_models_b200.simulation import _advanced
+    t, dt, want = np.float64(0.7), np.float64(0.1), np.float64(0.7)
+    for _ in range(1000):
+        want += dt
+    assert _advanced(t, dt, 1000) == want and _advanced(t, dt, 1) == t + dt
