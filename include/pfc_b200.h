@@ -174,6 +174,13 @@ int pfc_plan_info(pfc_plan* plan, int64_t* out16);
 /* OR-ed into a PFC_FLAG_ROW_EE / PFC_FLAG_COL_EE value: that pass's two-lane packed FP32
  * kernel (8 or 16 values per lane) */
 #define PFC_EE_PACKED 0x80
+/* OR-ed into a PFC_FLAG_ROW_EE value, or PFC_TILE_PAIRED into a PFC_FLAG_ROW_TILE value of 2, 4
+ * or 8: on power-of-two rows the plan takes the row kernel with paired butterflies, at its own
+ * values per thread, as it does when PFC_FLAG_ROW_EE and PFC_FLAG_ROW_TILE are 0. Where that
+ * kernel does not apply (nx/2 not a power of two, ny not whole tiles), and for the work queue,
+ * the rest of the variant counts. */
+#define PFC_TILE_PAIRED 16
+#define PFC_EE_PAIRED 0x40
 #define PFC_FLAG_ROW_EE(e) ((int32_t)(e) << 8)
 #define PFC_FLAG_COL_EE(e) ((int32_t)(e) << 16)
 #define PFC_FLAG_ROW_TILE(r) ((int32_t)(r) << 24)
@@ -185,8 +192,10 @@ int pfc_plan_info(pfc_plan* plan, int64_t* out16);
 #define PFC_FLAG_ROW_TILE_OF(f) (((f) >> 24) & 0x1f)
 #define PFC_FLAG_COL_CTA_OF(f) ((((f) >> 29) & 3) ? 1 << ((((f) >> 29) & 3) - 1) : 0)
 
-/* The variant a plan uses: out4 = {row values per thread, column values per thread,
- * row tile rows, 1 if the power-of-two step kernels are used} (zeros when not). */
+/* The variant a plan uses: out4 = {row values per thread (of the one-lane kernel where the plan
+ * pairs butterflies), column values per thread, row tile rows (with PFC_TILE_PAIRED where it
+ * does), kernels: 0 run-time kernels (the others 0 too), 1 one-lane or paired row, 2 packed, 3
+ * packed row, 4 packed column}. */
 int pfc_plan_variant(pfc_plan* plan, int32_t* out4);
 
 /* The step path of a plan: PFC_PATH_MIXED_RADIX (row and column kernels of any radix

@@ -32,6 +32,7 @@ STATUS_TIMEOUT = 2
 
 
 EE_PACKED = 0x80
+EE_PAIRED = 0x40
 PACKED_NONE, PACKED_BOTH, PACKED_ROW, PACKED_COL = 0, 1, 2, 3
 
 

@@ -100,6 +100,23 @@ std::vector<int> mixed_radices(int n, bool fp32) {
   return out;
 }
 
+// The tables [q - 1][k] of passes 1 and on of a compile-time sequence.
+void build_pass_tables(int n, const std::vector<int>& radices, const std::vector<long double>& root,
+                       std::vector<long double>& tw, int& off) {
+  off = (int)(tw.size() / 2);
+  int ns = radices[0];
+  for (size_t p = 1; p < radices.size(); ++p) {
+    const int R = radices[p];
+    for (int q = 1; q < R; ++q)
+      for (int k = 0; k < ns; ++k) {
+        const long long i = (long long)q * k * (n / (ns * R));
+        tw.push_back(root[2 * i]);
+        tw.push_back(root[2 * i + 1]);
+      }
+    ns *= R;
+  }
+}
+
 unsigned div_magic(int d) { return d == 1 ? 0u : (unsigned)((1ULL << 32) / (unsigned)d) + 1u; }
 
 // exp(-2 pi i k / n), k < n, in long double (each trigonometric value of a plan's tables is
@@ -162,6 +179,16 @@ int threads_per_fft(const std::vector<int>& radices, int n, bool fp32) {
 
 }  // namespace
 
+namespace {
+// Launch shape of the power-of-two row kernel (one side of the fast step).
+struct FastRowSide {
+  bool ok = false, packed = false, paired = false;
+  void* fn = nullptr;
+  int ee = 0, rows = 0, threads = 0, ld = 0, grid = 0, tw_a = 0, tw_b = 0, rt4 = 0;
+  size_t smem = 0;
+};
+}  // namespace
+
 struct pfc_plan {
   pfc_problem prob;
   int device = 0;
@@ -204,6 +231,8 @@ struct pfc_plan {
   int ee_row = 0, ee_col = 0;  // elements per thread of the fast kernels (per lane when packed)
   bool packed = false;         // two-lane packed FP32 step kernels (pfc_pack_step.cuh) on either pass
   bool packed_row = false, packed_col = false;
+  bool paired_row = false;     // row kernel with paired butterflies (pfc_rowpair.cuh)
+  FastRowSide one_row;         // the one-lane row kernel's shape, which the work-queue kernel runs
   // log PFC with an external potential (PFC_FLAG_EXTV, pfc_extv.cu)
   bool extv = false;
   pfc::ExtvState* extv_st = nullptr;   // device
@@ -419,13 +448,6 @@ bool fast_seq_tables(int lg, int ee, std::vector<long double>& tw, int& a, int& 
   return ee == 8 ? FastInst<double, 8>::tables(lg, tw, a, b) : FastInst<double, 16>::tables(lg, tw, a, b);
 }
 
-// Launch shape of the power-of-two row kernel (one side of the fast step).
-struct FastRowSide {
-  bool ok = false, packed = false;
-  void* fn = nullptr;
-  int ee = 0, rows = 0, threads = 0, ld = 0, grid = 0, tw_a = 0, tw_b = 0, rt4 = 0;
-  size_t smem = 0;
-};
 struct FastColSide {
   bool ok = false, packed = false;
   void* fn = nullptr;
@@ -475,6 +497,49 @@ int fast_row_side(pfc_plan* h, int ee, int tile, std::vector<long double>& tw, F
   o.ee = ee;
   if (lm >= 0) fast_seq_tables<T>(lm, ee, tw, o.tw_a, o.tw_b);
   else MixInst<T>::tables(h->m, tw, o.tw_a, o.tw_b);
+  o.ok = true;
+  return PFC_OK;
+}
+
+// Row kernel with paired butterflies (power-of-two rows, whole tiles): values per thread and
+// rows per tile by row length and precision, and the passes' tables of both sequences (one
+// copy when they run the same radices). `tile`: the variant's rows per CTA, or 0.
+// Rows of up to 512 points take 8 values a thread (the most threads; us per step on B200 with 8
+// / 16 values: 256^2 FP64 6.7 / 6.8, FP32 6.8 / 7.3, 512^2 8.0 / 8.5 and 7.4 / 8.7, 1024^2 log
+// 20.6 / 21.1 and 13.6 / 16.2), longer ones as many as 128 registers hold (2048^2 FP64 8 / 16
+// values 56.9 / 51.7, FP32 16 / 32 values 31.2 / 30.2, 8192^2 598 / 580). Tiles hold 64-byte
+// runs where a CTA of them fits an SM, and in FP32 32-byte ones for single plans of 256- and
+// 512-point rows, whose CTAs are few (512^2 7.4 against 7.7, 1024^2 log 13.6 against 14.2; a
+// batch of 24 512^2 plans prefers 8 rows, 41.3 against 43.1 us) and for 2048 points (121 against
+// 124). One-lane kernel at its tuned variants: 256^2 FP64 8.1, FP32 8.2; 512^2 9.2, 8.5; 1024^2
+// log 22.5, 14.8; 2048^2 59.3, 32.9; 4096^2 260, 138 (packed, TMA); 8192^2 1375, 615 (packed, TMA).
+template <class T>
+int pair_row_side(pfc_plan* h, int tile, std::vector<long double>& tw, FastRowSide& o) {
+  const int lm = ilog2_exact(h->m);
+  if (lm < 6) return PFC_OK;   // (a tile of 32-point rows is less than a warp)
+  int ee, rows;
+  if (sizeof(T) == 4) {
+    ee = lm <= 9 ? 8 : 32;
+    rows = (lm == 10 || (lm <= 9 && (tile >= 8 || (!tile && lm <= 7)))) ? 8 : 4;
+  } else {
+    ee = lm <= 9 ? 8 : 16;
+    rows = lm <= 11 ? 4 : 2;
+  }
+  PairKernel k;
+  if (h->ny % rows || !PairInst<T>::row(lm, ee, rows, h->prob.model, &k)) return PFC_OK;
+  const std::vector<long double> root = unit_roots(h->m);
+  std::vector<int> r = k.radices;
+  build_pass_tables(h->m, r, root, tw, o.tw_a);
+  std::reverse(r.begin(), r.end());
+  if (r == k.radices) o.tw_b = o.tw_a;
+  else build_pass_tables(h->m, r, root, tw, o.tw_b);
+  o.rows = rows;
+  o.threads = k.threads;
+  o.grid = h->ny / rows;
+  o.smem = k.smem;
+  o.fn = k.fn;
+  o.ee = ee;
+  o.paired = true;
   o.ok = true;
   return PFC_OK;
 }
@@ -610,7 +675,7 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   const bool row_packed = all_packed || (fr & PFC_EE_PACKED), col_packed = all_packed || (fc & PFC_EE_PACKED);
   if ((row_packed || col_packed) && sizeof(T) != 4)
     return fail(PFC_E_ARG, "pfc_plan_create: the packed kernels are built for the FP32-mixed form only");
-  const int er = fr & ~PFC_EE_PACKED, ec = fc & ~PFC_EE_PACKED;
+  const int er = fr & ~(PFC_EE_PACKED | PFC_EE_PAIRED), ec = fc & ~PFC_EE_PACKED;
   const int ee_r = er ? er : (row_packed ? 16 : fast_ee_default<T>());
   const int ee_c = ec ? ec : (col_packed ? 16 : fast_ee_default<T>());
   if (row_packed ? (ee_r != 8 && ee_r != 16) : !fast_ee_valid<T>(ee_r))
@@ -619,7 +684,13 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   if (col_packed ? (ee_c != 8 && ee_c != 16) : !fast_ee_valid<T>(ee_c))
     return fail(PFC_E_ARG, "pfc_plan_create: column kernel values per thread %d not built (FP32: 8, 16 or 32; "
                 "FP64: 8 or 16; packed: 8 or 16 per lane)", ee_c);
-  const int tile = PFC_FLAG_ROW_TILE_OF(flags);
+  int tile = PFC_FLAG_ROW_TILE_OF(flags);
+  // paired butterflies where the caller asks for them or leaves the row kernel to the plan
+  bool paired = (fr & PFC_EE_PAIRED) || (!fr && !tile && !all_packed);
+  if (tile == (PFC_TILE_PAIRED | 2) || tile == (PFC_TILE_PAIRED | 4) || tile == (PFC_TILE_PAIRED | 8)) {
+    paired = true;
+    tile &= ~PFC_TILE_PAIRED;
+  }
   if (tile && (tile > 16 || (row_packed && ((tile & (tile - 1)) || tile < 2))))
     return fail(PFC_E_ARG, "pfc_plan_create: row tile %d: at most 16 rows (packed: a power of two >= 2)", tile);
   if (flags & PFC_FLAG_GENERIC_ONLY) return PFC_OK;
@@ -628,6 +699,16 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   FastColSide c;
   int rc = row_packed ? pack_row_side(h, ee_r, tile, tw, r) : fast_row_side<T>(h, ee_r, tile, tw, r);
   if (rc) return rc;
+  if (!row_packed) h->one_row = r;
+  if (paired) {
+    FastRowSide q;
+    rc = pair_row_side<T>(h, tile, tw, q);
+    if (rc) return rc;
+    if (q.ok) {
+      q.ee = r.ok ? r.ee : q.ee;   // reported as the variant's
+      r = q;
+    }
+  }
   rc = col_packed ? pack_col_side(h, ee_c, col_cta, tw, c) : fast_col_side<T>(h, ee_c, col_cta, tw, c);
   if (rc) return rc;
   if (!r.ok || !c.ok) return PFC_OK;   // generic path
@@ -647,6 +728,7 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   h->tw_ca = c.tw_a; h->tw_cb = c.tw_b;
   h->rt4_off = r.rt4;
   h->packed_row = r.packed;
+  h->paired_row = r.paired;
   h->packed_col = c.packed;
   h->packed = r.packed || c.packed;
   if (int e = raise_smem_limit(h->fast_row_fn, h->fr_smem)) return e;
@@ -1671,8 +1753,9 @@ int pfc_plan_variant(pfc_plan* h, int32_t* o) {
   if (!h || !o) return fail(PFC_E_ARG, "pfc_plan_variant: null argument");
   o[0] = h->fast ? h->ee_row : 0;
   o[1] = h->fast ? h->ee_col : 0;
-  o[2] = h->fast ? h->fr_rows : 0;
-  // fast: 1 one-lane kernels, 2 packed row and column, 3 packed row only, 4 packed column only
+  o[2] = h->fast ? h->fr_rows | (h->paired_row ? PFC_TILE_PAIRED : 0) : 0;
+  // fast: 1 one-lane (or paired-row) kernels, 2 packed row and column, 3 packed row only, 4
+  // packed column only
   o[3] = !h->fast ? 0 : h->packed_row && h->packed_col ? 2 : h->packed_row ? 3 : h->packed_col ? 4 : 1;
   return PFC_OK;
 }
@@ -2079,15 +2162,17 @@ constexpr int kQueueItemsPerPass = 8;
 const char* queue_refusal(const pfc_plan* h) {
   const int lr = ilog2_exact(h->m), lc = ilog2_exact(h->ny);
   if (lr < 0 || lc < 0) return "the work-queue kernel steps power-of-two grids";
-  if (!h->fast || h->packed || h->onecta || h->extv) return "plans must use the one-lane power-of-two step kernels";
+  const FastRowSide& row = h->one_row;
+  if (!h->fast || h->packed || !row.ok || h->onecta || h->extv)
+    return "plans must use the one-lane power-of-two step kernels";
   if (h->prob.model != PFC_MODEL_STD) return "the work-queue kernel steps stdPFC plans";
   if (lr < kQueueMinLogRow || lr > kQueueMaxLogRow || lc < kQueueMinLogCol || lc > kQueueMaxLogCol)
     return "grid sides must be 64 .. 1024";
-  if (h->ee_row != queue_row_ee(!h->fp32, h->m) || h->ee_col != queue_col_ee(!h->fp32, h->ny))
+  if (row.ee != queue_row_ee(!h->fp32, h->m) || h->ee_col != queue_col_ee(!h->fp32, h->ny))
     return "the plan's values per thread differ from the work-queue kernel's";
-  if (h->fr_threads > kQueueThreads || h->fc_threads > kQueueThreads || h->fr_threads % 32 || h->fc_threads % 32)
+  if (row.threads > kQueueThreads || h->fc_threads > kQueueThreads || row.threads % 32 || h->fc_threads % 32)
     return "a pass's CTA is not whole warps of at most 256 threads";
-  if (h->fr_smem > kQueueSmemMax || h->fc_smem > kQueueSmemMax) return "a pass needs more than 48 KiB of shared memory";
+  if (row.smem > kQueueSmemMax || h->fc_smem > kQueueSmemMax) return "a pass needs more than 48 KiB of shared memory";
   return nullptr;
 }
 
@@ -2100,7 +2185,7 @@ int queue_build(pfc_queue* q) {
     int c = 0;
     for (; c < (int)q->classes.size(); ++c) {
       const pfc_plan* r = q->plans[q->classes[c][0]];
-      if (r->fast_row_fn == h->fast_row_fn && r->fast_col_fn == h->fast_col_fn && r->fr_rows == h->fr_rows &&
+      if (r->one_row.fn == h->one_row.fn && r->fast_col_fn == h->fast_col_fn && r->one_row.rows == h->one_row.rows &&
           r->fc_threads == h->fc_threads && r->nx == h->nx && r->ny == h->ny && r->prob.g == h->prob.g &&
           r->prob.clamp_log == h->prob.clamp_log && r->prob.min_phi == h->prob.min_phi)
         break;
@@ -2115,19 +2200,25 @@ int queue_build(pfc_queue* q) {
     const std::vector<int>& mem = q->classes[c];
     const pfc_plan* r = q->plans[mem[0]];
     QueueClass<T>& k = host[c];
+    const FastRowSide& row = r->one_row;
     k.row = fast_row_args<T>(r, nullptr);
+    k.row.rows = row.rows;
+    k.row.ld = row.ld;
+    k.row.rows_log2 = ilog2_exact(row.rows);
+    k.row.twA = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_a;
+    k.row.twB = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_b;
     k.col = fast_col_args<T>(r, nullptr);
     k.row_log = ilog2_exact(r->m);
     k.col_log = ilog2_exact(r->ny);
-    k.row_threads = r->fr_threads;
+    k.row_threads = row.threads;
     k.col_threads = r->fc_threads;
     // a few items per member and pass: each item pays one dependency check and one
     // completion, and a pass of more, smaller items gains little from the finer grain
-    k.row_group = std::max(1, r->fr_grid / kQueueItemsPerPass);
+    k.row_group = std::max(1, row.grid / kQueueItemsPerPass);
     k.col_group = std::max(1, r->fc_grid / kQueueItemsPerPass);
-    k.row_items = r->fr_grid / k.row_group;
+    k.row_items = row.grid / k.row_group;
     k.col_items = r->fc_grid / k.col_group;
-    q->smem = std::max(q->smem, std::max(r->fr_smem, r->fc_smem));
+    q->smem = std::max(q->smem, std::max(row.smem, r->fc_smem));
     for (int p = 0; p < 2; ++p) {
       std::vector<BatchBufs> tb(mem.size());
       for (size_t j = 0; j < mem.size(); ++j) {

@@ -42,6 +42,19 @@ struct FastInst {
   static bool tables(int lg, std::vector<long double>& tw, int& offA, int& offB);
 };
 
+// Power-of-two row step kernels with paired butterflies (pfc_rowpair.cuh): 2^lg-point rows, ee
+// values per thread, `rows` rows a CTA (64- or 32-byte runs).
+struct PairKernel {
+  void* fn = nullptr;
+  int threads = 0;
+  size_t smem = 0;
+  std::vector<int> radices;   // of sequence A
+};
+template <class T>
+struct PairInst {
+  static bool row(int lg, int ee, int rows, int model, PairKernel* out);
+};
+
 // Register-resident step kernels for transforms of N = ODD * 2^k points, ODD = 3, 5, 7
 // and k = kMixMinLog2 .. kMixMaxLog2 (pfc_fastmix_inst.cuh), by transform length.
 constexpr int kMixMinLog2 = 4, kMixMaxLog2 = 9;

@@ -375,7 +375,14 @@ def _kernel_flags(kernels, prob):
     as programmatic dependent launches, 2: the column kernel only) and "packed"
     (1: the two-lane packed FP32 kernels on both passes, 2: row pass only, 3: column pass
     only; ee_* of a packed pass count values per lane), "tma" (the packed row kernel's tile
-    staged by the tensor memory accelerator)."""
+    staged by the tensor memory accelerator). A tuned choice ("auto", or what `tune.lookup`
+    returns) takes the row kernel with paired butterflies on power-of-two rows, as a dict does
+    with "row_tile" 16 | rows (rows 2, 4 or 8) or without "ee_row" and "row_tile"."""
+    from . import tune
+    if kernels == "auto":
+        kernels = tune.lookup(prob.nx, prob.ny, prob.precision, prob.model) or "default"
+    if isinstance(kernels, tune.TunedVariant) and not kernels.get("generic"):
+        return _lib.flag_variant(**kernels) | (_lib.EE_PAIRED << 8)
     if isinstance(kernels, dict):
         return _lib.flag_variant(**{k: kernels.get(k, 0) for k in ("ee_row", "ee_col", "row_tile", "col_cta",
                                                                     "pdl", "packed", "tma", "generic")})
@@ -383,10 +390,6 @@ def _kernel_flags(kernels, prob):
         return _lib.FLAG_GENERIC_ONLY
     if kernels == "default":
         return 0
-    if kernels == "auto":
-        from . import tune
-        v = tune.lookup(prob.nx, prob.ny, prob.precision, prob.model)
-        return _lib.flag_variant(**v) if v else 0
     raise ValueError(f"kernels must be 'auto', 'default', 'generic' or a variant dict, got {kernels!r}")
 
 

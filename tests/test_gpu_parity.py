@@ -578,3 +578,34 @@ def test_long_odd_factor_sides_against_oracle(nx, ny, precision, model):
     o.set_field(ref)
     local = sim.plan.get_field(_lib.FIELD_LOCAL_N | _lib.FIELD_OF_CURRENT).cpu().numpy()
     assert rel_l2(local - f0.mean(), o.local_field() - f0.mean()) < tol
+
+
+@pytest.mark.parametrize("nx", [64, 128, 256, 512, 1024, 2048, 4096, 8192])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("model", ["std", "log"])
+def test_paired_row_kernels_match_the_runtime_kernels(nx, precision, model):
+    """The row kernel with paired butterflies, which plans take for power-of-two rows of at least
+    64 complex points, at every row length (and the one below) and tile height, on columns of 32 (one to sixteen tiles) and 96 sites, against
+    the run-time kernels: both round each transform to a few ulp, so 3 steps agree within 1e-13
+    (FP64) and 5e-6 of the deviation (FP32, about 80 ulp)."""
+    kw = dict(Gamma=1.0, beta=0.5, q0=1.0, epsilon=-0.9, g=-2.0, dt=0.05) if model == "log" else \
+        dict(Gamma=1.0, beta=1.0, q0=1.0, epsilon=-0.3, g=0.2, dt=0.3)
+    mean = 0.6 if model == "log" else -0.3
+    mod = logpfc if model == "log" else stdpfc
+    build = logpfc.BuildLogPFCModelParameters if model == "log" else stdpfc.BuildStdPFCModelParameters
+    for ny in (32, 96):
+        f0 = mean + 0.05 * np.random.default_rng(nx + ny).uniform(-1, 1, (ny, nx))
+        out = {}
+        for kernels in ("generic", "auto", {"row_tile": 16 | 4}, {"row_tile": 16 | 8}):
+            sim = mod.BuildB200_Simulation(build(**kw), mod.Build2DGeometry(nx, ny, nx * 0.8, ny * 0.8),
+                                           precision=precision, kernels=kernels, one_cta=False)
+            v = sim.plan.variant()
+            assert (v["row_tile"] & 16 != 0) == (kernels != "generic" and nx >= 128), (kernels, v)
+            (sim.State.phi if model == "log" else sim.State.n)[...] = f0
+            sim.TimeSteps(3)
+            out[str(kernels)] = (sim.State.phi if model == "log" else sim.State.n).get()
+            sim.plan.close()
+        ref = out.pop("generic")
+        tol = 1e-13 * np.linalg.norm(ref) if precision == "fp64" else 5e-6 * np.linalg.norm(ref - ref.mean())
+        for k, got in out.items():
+            assert np.linalg.norm(got - ref) <= tol, (ny, k)
