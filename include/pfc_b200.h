@@ -178,7 +178,9 @@ int pfc_plan_info(pfc_plan* plan, int64_t* out16);
  * or 8: on power-of-two rows the plan takes the row kernel with paired butterflies, at its own
  * values per thread, as it does when PFC_FLAG_ROW_EE and PFC_FLAG_ROW_TILE are 0. Where that
  * kernel does not apply (nx/2 not a power of two, ny not whole tiles), and for the work queue,
- * the rest of the variant counts. */
+ * the rest of the variant counts. With PFC_EE_PAIRED the plan also mixes kernels by pass: short
+ * odd-factor columns, and the side without a register-resident kernel beside a power-of-two one,
+ * run the run-time kernels. */
 #define PFC_TILE_PAIRED 16
 #define PFC_EE_PAIRED 0x40
 #define PFC_FLAG_ROW_EE(e) ((int32_t)(e) << 8)
@@ -206,9 +208,9 @@ int pfc_plan_variant(pfc_plan* plan, int32_t* out4);
 #define PFC_PATH_MIXED_RADIX 0
 #define PFC_PATH_POW2 1
 #define PFC_PATH_ONE_CTA 2
-#define PFC_PATH_FAST_MIXED 3   /* the register-resident step kernels on a grid whose sides
-                                   are N = ODD * 2^k (ODD = 3, 5, 7; 2^k = 16 .. 512) or
-                                   powers of two, not both powers of two */
+#define PFC_PATH_FAST_MIXED 3   /* register-resident kernels on one or both passes of a grid whose
+                                   sides are not both powers of two (for both: sides N = ODD *
+                                   2^k, ODD = 3, 5, 7, 2^k = 16 .. 512, or powers of two) */
 int pfc_plan_path(pfc_plan* plan, int32_t* path);
 
 /* Kernel launches issued by this plan since creation (for accounting). */

@@ -36,6 +36,12 @@ EE_PAIRED = 0x40
 PACKED_NONE, PACKED_BOTH, PACKED_ROW, PACKED_COL = 0, 1, 2, 3
 
 
+class TunedVariant(dict):
+    """A variant chosen for a plan rather than asked for (empty: no entry): on power-of-two rows
+    the plan takes its paired-butterfly row kernel (faster than every row variant the tuner
+    times, on every grid and batch measured), and it may run one pass on the run-time kernels."""
+
+
 def flag_variant(ee_row=0, ee_col=0, row_tile=0, col_cta=0, pdl=0, packed=0, tma=0, generic=0):
     """problem.flags bits selecting a step-kernel variant (PFC_FLAG_ROW_EE & co.).
     `packed`: 0 one-lane kernels, 1 the two-lane packed FP32 kernels on both passes,

@@ -129,6 +129,14 @@ __device__ __forceinline__ double nonlin_plain(double n, double g, int clamp, do
   return r;
 }
 
+// The log term near the singularity, in FP64. Out of line: the branch is rare, and its FP64
+// logarithm inlined for every value a thread holds (64 in the widest row kernel) overran the
+// instruction cache.
+static __device__ __noinline__ float nonlin_log_deep(float d, double inv_d, int clamp, double min_phi_rel, float log_min) {
+  const double xd = (double)d * inv_d;
+  return (clamp && !(1.0 + xd > min_phi_rel)) ? log_min : (float)log1p(xd);
+}
+
 // FP32 deviation form: N(mean + d) - N(mean). The log term is
 // log1p(d / mean); where 1 + d/mean < 1/8 it is evaluated in FP64.
 template <int MODEL>
@@ -138,12 +146,8 @@ __device__ __forceinline__ float nonlin_dev(float d, float c1, float c2, float i
   if (MODEL == kModelLog) {
     const float x = d * inv;
     float l;
-    if (x > -0.875f) {
-      l = log1pf(x);
-    } else {
-      const double xd = (double)d * inv_d;   // near-singular branch in FP64
-      l = (clamp && !(1.0 + xd > min_phi_rel)) ? log_min : (float)log1p(xd);
-    }
+    if (x > -0.875f) l = log1pf(x);
+    else l = nonlin_log_deep(d, inv_d, clamp, min_phi_rel, log_min);
     r += l;
   }
   return r;

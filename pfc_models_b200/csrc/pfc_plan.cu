@@ -223,8 +223,8 @@ struct pfc_plan {
   long long steps_since_set = 0;
   long long launches = 0;
   std::vector<double> hostA, hostBg;  // FP64 coefficients, (ny, m+1)
-  // specialised power-of-two step kernels (pfc_fast.cuh)
-  bool fast = false;
+  // register-resident step kernels (pfc_fast.cuh, pfc_rowpair.cuh), by pass; fast: on either
+  bool fast = false, fast_row = false, fast_col = false;
   void* fast_row_fn = nullptr;
   void* fast_col_fn = nullptr;
   int fr_rows = 0, fr_threads = 0, fr_ld = 0, fr_grid = 0;
@@ -511,19 +511,24 @@ int fast_row_side(pfc_plan* h, int ee, int tile, std::vector<long double>& tw, F
 // runs where a CTA of them fits an SM, and in FP32 32-byte ones for single plans of 256- and
 // 512-point rows, whose CTAs are few (512^2 7.4 against 7.7, 1024^2 log 13.6 against 14.2; a
 // batch of 24 512^2 plans prefers 8 rows, 41.3 against 43.1 us) and for 2048 points (121 against
-// 124). One-lane kernel at its tuned variants: 256^2 FP64 8.1, FP32 8.2; 512^2 9.2, 8.5; 1024^2
-// log 22.5, 14.8; 2048^2 59.3, 32.9; 4096^2 260, 138 (packed, TMA); 8192^2 1375, 615 (packed, TMA).
+// 124). The log model's logarithms, inlined per value, make the widest kernel's code long: 16
+// values for 1024 and 2048 points (2048^2 FP32 35.1 against 36.5, 4096^2 137 against 165; 8192^2
+// 690 against 687), and FP64 tiles of 2 rows at 2048 points (275 against 286). One-lane kernel
+// at its tuned variants: 256^2 FP64 8.1, FP32 8.2; 512^2 9.2, 8.5; 2048^2 59.3, 32.9; 4096^2
+// 260, 138 (packed, TMA); 8192^2 1375, 615 (packed, TMA); log 1024^2 22.5, 14.8, 2048^2 70.7,
+// 42.5, 4096^2 300, 174, 8192^2 FP32 780.
 template <class T>
 int pair_row_side(pfc_plan* h, int tile, std::vector<long double>& tw, FastRowSide& o) {
   const int lm = ilog2_exact(h->m);
   if (lm < 6) return PFC_OK;   // (a tile of 32-point rows is less than a warp)
+  const bool log = h->prob.model == PFC_MODEL_LOG;
   int ee, rows;
   if (sizeof(T) == 4) {
-    ee = lm <= 9 ? 8 : 32;
+    ee = lm <= 9 ? 8 : (log && lm <= 11) ? 16 : 32;
     rows = (lm == 10 || (lm <= 9 && (tile >= 8 || (!tile && lm <= 7)))) ? 8 : 4;
   } else {
     ee = lm <= 9 ? 8 : 16;
-    rows = lm <= 11 ? 4 : 2;
+    rows = lm <= (log ? 10 : 11) ? 4 : 2;
   }
   PairKernel k;
   if (h->ny % rows || !PairInst<T>::row(lm, ee, rows, h->prob.model, &k)) return PFC_OK;
@@ -662,6 +667,45 @@ int setup_tma(pfc_plan* h) {
   return raise_smem_limit(h->fast_row_fn, h->fr_smem);
 }
 
+// Odd-factor columns whose register-resident kernel (few threads holding ODD values each) is
+// slower than the run-time one. B200, column pass with its events, register-resident against
+// run-time, us: 3 x 128 FP32 20.3 / 12.7, FP64 14.0 / 11.8, 3 x 256 16.6 / 18.7 and 14.7 / 18.7;
+// 5 x 128 16.8 / 14.2 and 20.5 / 12.5, 5 x 256 22.4 / 25.9 and 33.9 / 29.1, 5 x 512 52.9 / 72.1 and
+// 90.2 / 96.3; 7 x 128 20.1 / 14.7 and 27.0 / 19.2, 7 x 256 26.7 / 34.8 and 58.7 / 46.4.
+bool short_odd_column(int ny, bool fp32) {
+  int odd = ny;
+  while (odd % 2 == 0) odd /= 2;
+  const int p2 = ny / odd;
+  return odd == 3 ? p2 < 256 : odd == 5 ? p2 < (fp32 ? 256 : 512) : p2 < (fp32 ? 256 : 512);
+}
+
+// FP64 rows of 7 x 32 points and more: 28 complex doubles a thread leave too few threads. Row
+// pass, register-resident against run-time, us: 7 x 32 21.2 / 13.0, 7 x 64 26.0 / 17.5, 7 x 128
+// 74 / 60 (7 x 16 16.5 / 11.4 keeps the register-resident kernel beside its columns).
+bool long_odd7_row(int m, bool fp32) { return !fp32 && m % 7 == 0 && m >= 7 * 32; }
+
+// Values per thread of a power-of-two column kernel by its length, as the tuned entries of
+// that length have it.
+template <class T> int column_ee(int ny) {
+  if (sizeof(T) == 4) return ny <= 1024 ? 8 : ny <= 4096 ? 16 : 32;
+  return ny <= 512 ? 8 : 16;
+}
+
+// Whether an FP64 plan takes the one-CTA step if its passes have no register-resident kernels:
+// grids whose rows and columns, each in two buffers, and state take up to kOneCtaMaxSmem (the
+// kernel itself holds the larger of rows and columns). Beyond that one CTA's threads take
+// longer than the launches it saves.
+int padded_length(int n) {   // of an exchange buffer: generic_pad and one, odd
+  const int ld = generic_pad(n - 1) + 2;
+  return ld % 2 ? ld : ld + 1;
+}
+bool onecta_fits(const pfc_plan* h) {
+  const size_t footprint =
+      (2 * ((size_t)h->ny * padded_length(h->m) + (size_t)h->m * padded_length(h->ny)) + h->nspec) * sizeof(double2);
+  return !h->fp32 && !(h->prob.flags & (PFC_FLAG_NO_ONE_CTA | PFC_FLAG_EXTV)) && h->ny <= kOneCtaMaxThreads &&
+         h->m <= kOneCtaMaxThreads && footprint <= kOneCtaMaxSmem;
+}
+
 // Chooses the fast kernels and their launch shapes; appends their twiddle tables to tw.
 // problem.flags may pick each kernel's values per thread (with PFC_EE_PACKED, or
 // PFC_FLAG_PACKED for both, the two-lane packed FP32 kernel of that pass), the row tile
@@ -677,7 +721,9 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
     return fail(PFC_E_ARG, "pfc_plan_create: the packed kernels are built for the FP32-mixed form only");
   const int er = fr & ~(PFC_EE_PACKED | PFC_EE_PAIRED), ec = fc & ~PFC_EE_PACKED;
   const int ee_r = er ? er : (row_packed ? 16 : fast_ee_default<T>());
-  const int ee_c = ec ? ec : (col_packed ? 16 : fast_ee_default<T>());
+  // a column kernel left to the plan without a tuned entry: as the entries of its length have it
+  const bool own_col = (fr & PFC_EE_PAIRED) && !fc && !col_packed;
+  const int ee_c = ec ? ec : (col_packed ? 16 : own_col ? column_ee<T>(h->ny) : fast_ee_default<T>());
   if (row_packed ? (ee_r != 8 && ee_r != 16) : !fast_ee_valid<T>(ee_r))
     return fail(PFC_E_ARG, "pfc_plan_create: row kernel values per thread %d not built (FP32: 8, 16 or 32; "
                 "FP64: 8 or 16; packed: 8 or 16 per lane)", ee_r);
@@ -694,7 +740,9 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   if (tile && (tile > 16 || (row_packed && ((tile & (tile - 1)) || tile < 2))))
     return fail(PFC_E_ARG, "pfc_plan_create: row tile %d: at most 16 rows (packed: a power of two >= 2)", tile);
   if (flags & PFC_FLAG_GENERIC_ONLY) return PFC_OK;
-  const int col_cta = PFC_FLAG_COL_CTA_OF(flags);
+  int col_cta = PFC_FLAG_COL_CTA_OF(flags);
+  if (own_col && !col_cta)   // fewer columns a CTA where that spreads them over more SMs or they are long
+    for (col_cta = 4; col_cta > 1 && (h->m / col_cta < 256 || (size_t)col_cta * h->ny * h->elt > 64 * 1024);) col_cta /= 2;
   FastRowSide r;
   FastColSide c;
   int rc = row_packed ? pack_row_side(h, ee_r, tile, tw, r) : fast_row_side<T>(h, ee_r, tile, tw, r);
@@ -711,7 +759,19 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   }
   rc = col_packed ? pack_col_side(h, ee_c, col_cta, tw, c) : fast_col_side<T>(h, ee_c, col_cta, tw, c);
   if (rc) return rc;
-  if (!r.ok || !c.ok) return PFC_OK;   // generic path
+  // A plan that chooses its kernels itself mixes them by pass: the run-time column kernel for
+  // short odd-factor columns, and a power-of-two side's kernel beside a side without one.
+  const bool row2 = ilog2_exact(h->m) >= 0, col2 = ilog2_exact(h->ny) >= 0;
+  const bool split = (fr & PFC_EE_PAIRED) && !onecta_fits(h);
+  const bool drop_row = split && r.ok && !row2 && long_odd7_row(h->m, sizeof(T) == 4);
+  const bool drop_col = split && c.ok && !c.packed && !col2 && short_odd_column(h->ny, sizeof(T) == 4);
+  r.ok = r.ok && !drop_row;
+  c.ok = c.ok && !drop_col;
+  if (!r.ok && !c.ok) return PFC_OK;   // run-time kernels
+  if (!c.ok && !drop_col && !(split && r.paired)) return PFC_OK;
+  if (!r.ok && !drop_row && !(split && col2 && h->ny >= 256)) return PFC_OK;
+  h->fast_row = r.ok;
+  h->fast_col = c.ok;
   h->fr_rows = r.rows;
   h->fr_threads = r.threads;
   h->fr_ld = r.ld;
@@ -731,9 +791,11 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   h->paired_row = r.paired;
   h->packed_col = c.packed;
   h->packed = r.packed || c.packed;
-  if (int e = raise_smem_limit(h->fast_row_fn, h->fr_smem)) return e;
-  if (int e = raise_smem_limit(h->fast_col_fn, h->fc_smem)) return e;
-  h->fast = true;
+  if (r.ok)
+    if (int e = raise_smem_limit(h->fast_row_fn, h->fr_smem)) return e;
+  if (c.ok)
+    if (int e = raise_smem_limit(h->fast_col_fn, h->fc_smem)) return e;
+  h->fast = r.ok || c.ok;
   return PFC_OK;
 }
 
@@ -819,7 +881,7 @@ FastColArgs<T> fast_col_args(const pfc_plan* h, const BatchBufs* table) {
 
 template <class T>
 int launch_step_row(pfc_plan* h, cudaStream_t s, const BatchBufs* table = nullptr, int count = 1) {
-  if (h->fast) {
+  if (h->fast_row) {
     FastRowArgs<T> a = fast_row_args<T>(h, table);
     void* args_pk[] = {(void*)&a, (void*)&h->tmap};
     void* args1[] = {(void*)&a};
@@ -850,7 +912,7 @@ int launch_step_row(pfc_plan* h, cudaStream_t s, const BatchBufs* table = nullpt
 // One column pass of a step: V, n_hat[cur] -> n_hat[cur ^ 1], W (batched as above).
 template <class T>
 int launch_step_col(pfc_plan* h, cudaStream_t s, const BatchBufs* table = nullptr, int count = 1) {
-  if (h->fast) {
+  if (h->fast_col) {
     FastColArgs<T> a = fast_col_args<T>(h, table);
     void* args[] = {(void*)&a};
     cudaError_t e = launch_step_kernel(h, h->fast_col_fn, dim3(h->fc_grid, count), dim3(h->fc_threads), args,
@@ -950,18 +1012,14 @@ int max_butterflies(const FftDesc& d) {
 // two-kernel step.
 int setup_onecta(pfc_plan* h) {
   h->onecta = false;
-  if (h->fp32 || h->fast || (h->prob.flags & PFC_FLAG_NO_ONE_CTA)) return PFC_OK;
+  if (h->fast) return PFC_OK;
   const int rset = onecta_rset(h->row_rset, h->col_rset);
   if (rset < 0 || !onecta_supported(rset)) return PFC_OK;
   // one thread per butterfly of the widest pass, at most a block
   const int items = std::max(h->ny * max_butterflies(h->rowfft), h->m * max_butterflies(h->colfft));
   const int threads = std::min((items + 31) / 32 * 32, kOneCtaMaxThreads);
   const size_t smem = onecta_smem_bytes(h->m, h->ny, h->row_ld, h->col_ld);
-  // grids whose rows and columns, each in two buffers, and state take up to kOneCtaMaxSmem (the
-  // kernel itself holds the larger of rows and columns): beyond that one CTA's threads
-  // take longer than the launches it saves
-  const size_t footprint = (2 * ((size_t)h->ny * h->row_ld + (size_t)h->m * h->col_ld) + h->nspec) * sizeof(double2);
-  if (h->ny > kOneCtaMaxThreads || h->m > kOneCtaMaxThreads || footprint > kOneCtaMaxSmem) return PFC_OK;
+  if (!onecta_fits(h)) return PFC_OK;
   if (smem > 48 * 1024) {
     cudaError_t e = onecta_allow_smem(kOneCtaMaxSmem);
     if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
@@ -1422,7 +1480,7 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
   std::vector<long double> tw;
   // two buffers of one padded transform fit an SM's shared memory: the two-buffer kernels,
   // both radix orders; longer transforms: the one-buffer kernels
-  auto padded = [](int n) { const int ld = generic_pad(n - 1) + 2; return ld % 2 ? ld : ld + 1; };
+  auto padded = padded_length;
   const bool row_two = 2 * (size_t)padded(m) * h->elt <= kMixedSmem;
   const bool col_two = 2 * (size_t)padded(p->ny) * h->elt <= kMixedSmem;
   auto plan_fft = [&](int n, bool two, const std::vector<int>& one, FftDesc& d, FftDesc& db) {
@@ -1449,7 +1507,7 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
     if (rc) return cleanup_fail(rc);
   }
 
-  if (!h->fp32 && !h->fast && !(p->flags & (PFC_FLAG_NO_ONE_CTA | PFC_FLAG_EXTV))) {
+  if (!h->fast && onecta_fits(h)) {
     h->dense = dense_shape(m, p->ny, h->dense_args) <= kOneCtaMaxSmem &&
                dense_products(h->dense_args) <= kDenseMaxProducts;
     if (h->dense) {
@@ -1751,9 +1809,9 @@ int64_t pfc_launch_count(pfc_plan* h) { return h ? h->launches : 0; }
 
 int pfc_plan_variant(pfc_plan* h, int32_t* o) {
   if (!h || !o) return fail(PFC_E_ARG, "pfc_plan_variant: null argument");
-  o[0] = h->fast ? h->ee_row : 0;
-  o[1] = h->fast ? h->ee_col : 0;
-  o[2] = h->fast ? h->fr_rows | (h->paired_row ? PFC_TILE_PAIRED : 0) : 0;
+  o[0] = h->fast_row ? h->ee_row : 0;
+  o[1] = h->fast_col ? h->ee_col : 0;
+  o[2] = h->fast_row ? h->fr_rows | (h->paired_row ? PFC_TILE_PAIRED : 0) : 0;
   // fast: 1 one-lane (or paired-row) kernels, 2 packed row and column, 3 packed row only, 4
   // packed column only
   o[3] = !h->fast ? 0 : h->packed_row && h->packed_col ? 2 : h->packed_row ? 3 : h->packed_col ? 4 : 1;
@@ -1790,7 +1848,7 @@ int pfc_batch_create(pfc_plan* const* plans, int32_t count, pfc_batch** out) {
       const pfc_plan* r = c.plans[0];
       // (mixed-radix plans of one size and precision share the FFT description, twiddle
       // tables and launch shape, all of which come from plans[0] of the class)
-      if (r->fast == h->fast && r->onecta == h->onecta && r->fast_row_fn == h->fast_row_fn &&
+      if (r->fast_row == h->fast_row && r->fast_col == h->fast_col && r->onecta == h->onecta && r->fast_row_fn == h->fast_row_fn &&
           r->fast_col_fn == h->fast_col_fn && r->packed_row == h->packed_row && r->fr_rows == h->fr_rows &&
           r->fc_threads == h->fc_threads &&
           r->row_rset == h->row_rset && r->col_rset == h->col_rset && r->prob.model == h->prob.model &&
@@ -2163,7 +2221,7 @@ const char* queue_refusal(const pfc_plan* h) {
   const int lr = ilog2_exact(h->m), lc = ilog2_exact(h->ny);
   if (lr < 0 || lc < 0) return "the work-queue kernel steps power-of-two grids";
   const FastRowSide& row = h->one_row;
-  if (!h->fast || h->packed || !row.ok || h->onecta || h->extv)
+  if (!h->fast_row || !h->fast_col || h->packed || !row.ok || h->onecta || h->extv)
     return "plans must use the one-lane power-of-two step kernels";
   if (h->prob.model != PFC_MODEL_STD) return "the work-queue kernel steps stdPFC plans";
   if (lr < kQueueMinLogRow || lr > kQueueMaxLogRow || lc < kQueueMinLogCol || lc > kQueueMaxLogCol)

@@ -378,10 +378,10 @@ def _kernel_flags(kernels, prob):
     staged by the tensor memory accelerator). A tuned choice ("auto", or what `tune.lookup`
     returns) takes the row kernel with paired butterflies on power-of-two rows, as a dict does
     with "row_tile" 16 | rows (rows 2, 4 or 8) or without "ee_row" and "row_tile"."""
-    from . import tune
     if kernels == "auto":
-        kernels = tune.lookup(prob.nx, prob.ny, prob.precision, prob.model) or "default"
-    if isinstance(kernels, tune.TunedVariant) and not kernels.get("generic"):
+        from . import tune
+        kernels = tune.lookup(prob.nx, prob.ny, prob.precision, prob.model) or _lib.TunedVariant()
+    if isinstance(kernels, _lib.TunedVariant) and not kernels.get("generic"):
         return _lib.flag_variant(**kernels) | (_lib.EE_PAIRED << 8)
     if isinstance(kernels, dict):
         return _lib.flag_variant(**{k: kernels.get(k, 0) for k in ("ee_row", "ee_col", "row_tile", "col_cta",

@@ -35,14 +35,6 @@ COL_CTA_CHOICES = (1, 2, 4)
 VARIANT_KEYS = ("ee_row", "ee_col", "row_tile", "col_cta", "pdl", "packed", "tma", "generic")
 PACKED_EE = (8, 16)                 # values per lane of the two-lane packed FP32 kernels
 PACKED_TILES = (2, 4, 8, 16)
-
-
-class TunedVariant(dict):
-    """A variant chosen for a plan rather than asked for: on power-of-two rows the plan takes
-    its paired-butterfly row kernel (faster than every row variant timed here, on every grid
-    and batch measured) and the entry's choice of the rest."""
-
-
 _lock = threading.Lock()
 _memo: dict = {}
 
@@ -92,7 +84,7 @@ def lookup(nx, ny, precision, model, device_name=None, batched=False):
         for path in (cache_path(), PACKAGED):
             e = _load(path).get(key)
             if e:
-                return TunedVariant({k: int(e.get(k) or 0) for k in VARIANT_KEYS})
+                return _lib.TunedVariant({k: int(e.get(k) or 0) for k in VARIANT_KEYS})
     return None
 
 
@@ -321,7 +313,7 @@ def refine(nx, ny, precision, model, base, batch=1, min_gain=0.01):
         generic_us, _ = _time_blocks(nx, ny, precision, model, {"generic": 1}, batch, fast=False)
     for cc in (0,) + COL_CTA_CHOICES:
         for pdl in (0, 1, 2):   # 2: the column kernel only
-            us, threads = _time_blocks(nx, ny, precision, model, TunedVariant(v0, col_cta=cc, pdl=pdl), batch,
+            us, threads = _time_blocks(nx, ny, precision, model, _lib.TunedVariant(v0, col_cta=cc, pdl=pdl), batch,
                                        skip=lambda th: (th, pdl) in seen)
             if threads is None:
                 return {"col_cta": 0, "pdl": 0}

@@ -609,3 +609,32 @@ def test_paired_row_kernels_match_the_runtime_kernels(nx, precision, model):
         tol = 1e-13 * np.linalg.norm(ref) if precision == "fp64" else 5e-6 * np.linalg.norm(ref - ref.mean())
         for k, got in out.items():
             assert np.linalg.norm(got - ref) <= tol, (ny, k)
+
+
+@pytest.mark.parametrize("nx,ny", [(448, 96), (224, 224), (896, 640), (256, 84), (840, 256), (60, 256), (1536, 768),
+                                   (128, 66)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_plans_that_mix_kernels_by_pass(nx, ny, precision):
+    """Plans that choose their own kernels run short odd-factor columns, and a side without a
+    register-resident kernel beside a power-of-two one, on the run-time kernels: against the
+    run-time kernels on both passes (19 steps: 1e-12 in FP64, 2e-5 of the deviation in FP32, as the
+    size tests), alone and in a batch."""
+    from pfc_models_b200.simulation import Batch
+    prm = stdpfc.BuildStdPFCModelParameters(Gamma=1.0, beta=1.0, q0=1.0, epsilon=-0.3, g=0.2, dt=0.3)
+    geom = stdpfc.Build2DGeometry(nx, ny, nx * 0.8, ny * 0.8)
+    f0 = -0.3 + 0.05 * np.random.default_rng(nx + ny).uniform(-1, 1, (ny, nx))
+    sims = [stdpfc.BuildB200_Simulation(prm, geom, precision=precision, kernels=k, one_cta=False)
+            for k in ("generic", "auto", "auto")]
+    for s in sims:
+        s.State.n[...] = f0
+    for s in sims[:2]:
+        s.TimeSteps(19)
+    b = Batch(sims[2:])
+    b.step(19)
+    ref, got, batched = [s.State.n.get() for s in sims]
+    tol = 1e-12 * np.linalg.norm(ref) if precision == "fp64" else 2e-5 * np.linalg.norm(ref - ref.mean())
+    assert np.linalg.norm(got - ref) <= tol
+    assert np.array_equal(got, batched)
+    b.close()
+    for s in sims:
+        s.plan.close()
