@@ -17,6 +17,7 @@
 // FP32_MIXED runs the same kernels on delta = n - mean in float; the mean is an
 // FP64 device scalar and the packed DC of delta_hat is held at exactly zero.
 #pragma once
+#include "pfc_extv.h"
 #include "pfc_fft.cuh"
 
 namespace pfc {
@@ -234,6 +235,7 @@ struct RowArgs {
   const double* add;        // materialise: constant added (device pointer), may be null
   double* partials;         // per-CTA compensated sums
   double* minmax;           // step mode, FP64 form: per-CTA (min, max) of the field, or null
+  ExtvState* extv;          // two-buffer kernels, with minmax: the last CTA decides M here, or null
   int clamp;
   double g, min_phi, min_log, epsilon;
   const BatchBufs* batch;   // step or reduce mode of a batch: per-plan W, V and scalars at [blockIdx.y]
@@ -264,6 +266,8 @@ struct ColArgs {
   const cplx<T>* coef;          // (A - 1, Bg) [kx][ky], kx <= m, ky <= ny/2, working precision
   const cplx<double>* coef64;   // FP32 form: the same in FP64, read for the slow modes
   const cplx<double>* forcing;  // step mode, FP64 form: added to n_hat', [kx][ky] (kx <= m), or null
+  const ExtvState* extv;        // two-buffer kernels: M's state; when it changed, the CTAs rebuild their
+  const ExtvCoefArgs* ec;       //   columns by these (in device memory), or null
   float slow_tau;
   double* partials;
   double* out_c128;             // export: (ny, m+1) complex128

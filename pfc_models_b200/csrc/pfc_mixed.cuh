@@ -227,6 +227,31 @@ __device__ __forceinline__ void packed_update(cplx<double> pk, cplx<double> pkp,
   okp = conj(h0n) + mul_i(conj(hmn));
 }
 
+// The external-potential decision by the row pass itself: the CTA that stores the last of the
+// ranges reduces them all and applies the reference's rules (a kernel of its own cost 3.2 us
+// and a launch gap a step). Out of line; every thread of the CTA calls it.
+static __device__ __noinline__ void extv_decide_last(const double* minmax, int nparts, ExtvState* st, double g) {
+  __shared__ bool last;
+  __shared__ double range[2];
+  if (threadIdx.x == 0) {
+    __threadfence();   // this CTA's pair before the count
+    last = atomicAdd(&st->done, 1u) == (unsigned)nparts - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double lo = INFINITY, hi = -INFINITY;
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
+    lo = fmin(lo, __ldcg(minmax + 2 * i));
+    hi = fmax(hi, __ldcg(minmax + 2 * i + 1));
+  }
+  block_minmax_store(lo, hi, range);
+  if (threadIdx.x == 0) {
+    extv_apply(st, range[0], range[1], g);
+    st->done = 0;
+  }
+}
+
 // ---------------------------------------------------------------- row kernel
 // `rows` = 2^rows_log2 rows per CTA, two buffers of rows * ld values. Modes as row_kernel's
 // (pfc_kernels.cuh).
@@ -344,7 +369,10 @@ __global__ void __launch_bounds__(256, 2) mixed_row_kernel(RowArgs<T> a) {
     mixed_switch<RSET, T>(a.fft.radix[np - 1], [&](auto r) {
       mixed_mid_items<decltype(r)::value, true, T>(a.fft, 0, rows, a.tw, ld_s, fn, st_s);
     });
-    if (sizeof(T) == 8 && a.minmax) block_minmax_store(lo, hi, a.minmax + 2 * blockIdx.x);
+    if (sizeof(T) == 8 && a.minmax) {
+      block_minmax_store(lo, hi, a.minmax + 2 * blockIdx.x);
+      if (MODEL == kModelLog && a.extv) extv_decide_last(a.minmax, gridDim.x, a.extv, a.g);
+    }
     flip();
     for (int p = 1; p < np; ++p) {
       mixed_pass<false, RSET, T>(a.fft_b, p, rows, a.tw, ld_s, st_s);
@@ -575,6 +603,14 @@ __global__ void __launch_bounds__(256, 2) mixed_col_kernel(ColArgs<T> a) {
     else
       l2_prefetch_range(reinterpret_cast<const void*>(k0 & lim), (unsigned)((k1 & lim) - (k0 & lim)),
                         threadIdx.x - half, blockDim.x - half);
+  }
+  if constexpr (MODE == kColStep && sizeof(T) == 8) {
+    if (a.extv && a.extv->changed) {   // M or V changed: this CTA's coefficients and forcing
+      const double M = a.extv->M;
+      for (int c = 0; c < cols; ++c) extv_rebuild_column(*a.ec, M, c0 + c);
+      if (c0 == 0) extv_rebuild_column(*a.ec, M, m);
+      __syncthreads();
+    }
   }
   // The CTA with the packed column, whose update pairs ky with ny - ky, parks its spectra in
   // shared memory between the two transforms; the others update in the middle pass.

@@ -236,6 +236,7 @@ struct pfc_plan {
   // log PFC with an external potential (PFC_FLAG_EXTV, pfc_extv.cu)
   bool extv = false;
   pfc::ExtvState* extv_st = nullptr;   // device
+  pfc::ExtvCoefArgs* extv_ec = nullptr;   // device: the rebuild's arguments
   double* extv_minmax = nullptr;       // per row-CTA (min, max) of the field
   double2* vhat = nullptr;             // rfft2 of V, (ny, m + 1)
   double2* forcing = nullptr;          // B lap V_hat, [kx][ky]
@@ -835,7 +836,11 @@ ExtvCoefArgs extv_coef_args(const pfc_plan* h) {
 
 // launches of one step of this plan (row and column kernels, plus the external-potential
 // decision and coefficient kernels)
-int launches_per_step(const pfc_plan* h) { return h->extv ? 4 : 2; }
+// (which are parts of the two-buffer kernels, launches of their own beside one-buffer ones)
+bool one_buffer(int rset) { return rset == kRadixPow2Big || rset == kRadixSmallBig; }
+int launches_per_step(const pfc_plan* h) {
+  return 2 + (h->extv && one_buffer(h->row_rset)) + (h->extv && one_buffer(h->col_rset));
+}
 
 // Arguments of the fast row kernel for plan h (a batch's members from `table`).
 template <class T>
@@ -900,11 +905,19 @@ int launch_step_row(pfc_plan* h, cudaStream_t s, const BatchBufs* table = nullpt
   // external potential: the field's range, the M decision and (when M or V changed) the
   // coefficients and the forcing, before the column pass
   ra.minmax = h->extv_minmax;
+  const bool own = one_buffer(h->row_rset);
+  if (!own) ra.extv = h->extv_st;
   int rc = launch_row<T, kRowStep>(h, ra, s, count);
   if (rc) return rc;
-  cudaError_t e = launch_extv_decide(h->extv_minmax, h->row_grid, h->extv_st, h->prob.g, s);
-  if (e == cudaSuccess) e = launch_extv_coef(extv_coef_args(h), h->extv_st, s);
-  h->launches += 2;
+  cudaError_t e = cudaSuccess;
+  if (own) {
+    e = launch_extv_decide(h->extv_minmax, h->row_grid, h->extv_st, h->prob.g, s);
+    ++h->launches;
+  }
+  if (e == cudaSuccess && one_buffer(h->col_rset)) {
+    e = launch_extv_coef(extv_coef_args(h), h->extv_st, s);
+    ++h->launches;
+  }
   if (e != cudaSuccess) return fail(PFC_E_CUDA, "external-potential step launch failed: %s", cudaGetErrorString(e));
   return PFC_OK;
 }
@@ -929,7 +942,13 @@ int launch_step_col(pfc_plan* h, cudaStream_t s, const BatchBufs* table = nullpt
   ca.nin_lo = static_cast<const cplx<float>*>(h->nhat_lo[h->cur]);
   ca.nout_lo = static_cast<cplx<float>*>(h->nhat_lo[h->cur ^ 1]);
   ca.batch = table;
-  if (h->extv) ca.forcing = reinterpret_cast<const cplx<double>*>(h->forcing);
+  if (h->extv) {
+    ca.forcing = reinterpret_cast<const cplx<double>*>(h->forcing);
+    if (!one_buffer(h->col_rset)) {
+      ca.extv = h->extv_st;
+      ca.ec = h->extv_ec;
+    }
+  }
   return launch_col<T, kColStep>(h, ca, s, count);
 }
 
@@ -1652,6 +1671,9 @@ int pfc_plan_create(const pfc_problem* p, pfc_plan** out) {
       st.ceil_tol = 0.1;
       st.min_phi = p->min_phi;
       e = cudaMemcpy(h->extv_st, &st, sizeof(st), cudaMemcpyHostToDevice);
+      const ExtvCoefArgs ec = extv_coef_args(h);
+      if (e == cudaSuccess) e = cudaMalloc(&h->extv_ec, sizeof(ec));
+      if (e == cudaSuccess) e = cudaMemcpy(h->extv_ec, &ec, sizeof(ec), cudaMemcpyHostToDevice);
     }
   }
   if (e != cudaSuccess)
@@ -1709,7 +1731,7 @@ int pfc_plan_destroy(pfc_plan* h) {
   for (void* p : {h->nhat[0], h->nhat[1], h->nhat_lo[0], h->nhat_lo[1], h->W, h->V, h->W2, h->coef, h->coef64, h->tw})
     if (p) cudaFree(p);
   if (h->partials) cudaFree(h->partials);
-  for (void* q : {(void*)h->extv_st, (void*)h->extv_minmax, (void*)h->vhat, (void*)h->forcing, h->scratch_state})
+  for (void* q : {(void*)h->extv_st, (void*)h->extv_ec, (void*)h->extv_minmax, (void*)h->vhat, (void*)h->forcing, h->scratch_state})
     if (q) cudaFree(q);
   if (h->scal) cudaFree(h->scal);
   if (h->status) cudaFree(h->status);

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include "pfc_extv.h"
+
 namespace pfc {
 
 // Radix-set codes of the run-time kernels: kRadixPow2, kRadixSmall and kRadixAll
@@ -145,23 +147,8 @@ cudaError_t dense_allow_smem(size_t bytes);
 cudaError_t launch_dense_step(const DenseArgs& args, const BatchBufs* table, int count, long long nsteps, int model,
                               size_t smem, cudaStream_t stream);
 
-// Log PFC with an external potential (pfc_extv.cu): the state of the M shift, kept in
-// device memory, and the arguments of the coefficient rebuild.
-struct ExtvState {
-  double M, phi_min, phi_max;   // shift and the range it was optimised for
-  double floor_tol, ceil_tol;   // relative tolerances of ValidatePhiRange (0.1, 0.1)
-  double min_phi;               // replaces a non-positive minimum in OptimizeM
-  double last_min, last_max;    // the field's range seen by the last step
-  int init, changed, count;
-  int v_dirty;                  // nonzero: V changed since the forcing was built
-};
-struct ExtvCoefArgs {
-  int nx, ny, m, nyh;
-  double fx, fy, gamma, beta, q0, epsilon, dt, small_z_tol;
-  double2* coef;          // (A - 1 - M Bg, Bg), [kx][ky <= ny/2]
-  const double2* vhat;    // rfft2 of V, (ny, m + 1) row-major
-  double2* forcing;       // B lap V_hat, [kx][ky], kx <= m
-};
+// Log PFC with an external potential (pfc_extv.cu): the decision and the rebuild as kernels of
+// their own, for plans whose row or column pass runs the one-buffer kernels.
 cudaError_t launch_extv_decide(const double* minmax, int nparts, ExtvState* st, double g, cudaStream_t s);
 cudaError_t launch_extv_coef(const ExtvCoefArgs& a, const ExtvState* st, cudaStream_t s);
 

@@ -81,3 +81,39 @@ def test_extv_refuses_other_forms():
     dv = torch.as_tensor(v, device="cuda")
     with pytest.raises(_lib.PfcError):
         _lib.check(sim.plan.lib.pfc_set_potential(sim.plan.handle, dv.data_ptr(), None))
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 48), (44, 26), (22, 5), (16, 8192), (16384, 6)])
+def test_extv_decision_and_rebuild_by_kernel_form(nx, ny):
+    """The decision in the row pass's last CTA and the rebuild in the column CTAs (two-buffer
+    kernels: one CTA, several, single-pass columns) and their own kernels beside one-buffer
+    transforms (8192 points), against the oracle's restatement: a field that grows through its
+    tolerances re-optimises M several times, and a new potential rebuilds the forcing alone.
+    FP64, 12 steps: M and the field within 1e-11 (a few ulp a step, amplified by 1 / (max - min)
+    in M)."""
+    from oracle import pfc_oracle as orc
+    lx, ly = nx * 0.9, ny * 0.8
+    rng = np.random.default_rng(nx + ny)
+    x = np.arange(nx) * 0.9
+    f0 = 0.55 + 0.05 * np.cos(2 * np.pi * x / lx)[None, :] + 0.02 * rng.uniform(-1, 1, (ny, nx))
+    V1 = 0.05 * rng.uniform(-1, 1, (ny, nx))
+    V2 = 0.3 * rng.uniform(-1, 1, (ny, nx))
+    kw = dict(Gamma=1.0, beta=0.5, q0=1.0, epsilon=-0.9, g=-2.0, dt=0.05)
+    o = orc.OracleExtv(orc.Params(smallZTol=1e-8, **kw), orc.build_geometry(nx, ny, lx, ly), V=V1)
+    o.set_field(f0)
+    prm = logpfc_extv.BuildLogPFCModel_withVacancyForce_Parameters(**kw)
+    sim = logpfc_extv.BuildB200_Simulation(prm, logpfc_extv.BuildGeometry(nx, ny, lx, ly))
+    sim.State.phi[...] = f0
+    sim._externalV.SetPotential(1.0, V1)
+    for step in range(12):
+        if step == 6:
+            o.V_hat = np.fft.rfft2(V2)
+            sim._externalV.SetPotential(1.0, V2)
+        o.step()
+        sim.TimeStep()
+        assert sim.State.M == pytest.approx(o.M, rel=1e-11), step
+        assert sim.State.optimizations == o.optimizations, step
+    assert o.optimizations >= (2 if nx * ny > 200 else 1)   # (a few sites stay within the tolerances)
+    got = sim.State.phi.get()
+    assert np.linalg.norm(got - o.n) <= 1e-11 * np.linalg.norm(o.n)
+    sim.plan.close()
