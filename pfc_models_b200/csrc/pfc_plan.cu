@@ -502,37 +502,17 @@ int fast_row_side(pfc_plan* h, int ee, int tile, std::vector<long double>& tw, F
   return PFC_OK;
 }
 
-// Row kernel with paired butterflies (power-of-two rows, whole tiles): values per thread and
-// rows per tile by row length and precision, and the passes' tables of both sequences (one
-// copy when they run the same radices). `tile`: the variant's rows per CTA, or 0.
-// Rows of up to 512 points take 8 values a thread (the most threads; us per step on B200 with 8
-// / 16 values: 256^2 FP64 6.7 / 6.8, FP32 6.8 / 7.3, 512^2 8.0 / 8.5 and 7.4 / 8.7, 1024^2 log
-// 20.6 / 21.1 and 13.6 / 16.2), longer ones as many as 128 registers hold (2048^2 FP64 8 / 16
-// values 56.9 / 51.7, FP32 16 / 32 values 31.2 / 30.2, 8192^2 598 / 580). Tiles hold 64-byte
-// runs where a CTA of them fits an SM, and in FP32 32-byte ones for single plans of 256- and
-// 512-point rows, whose CTAs are few (512^2 7.4 against 7.7, 1024^2 log 13.6 against 14.2; a
-// batch of 24 512^2 plans prefers 8 rows, 41.3 against 43.1 us) and for 2048 points (121 against
-// 124). The log model's logarithms, inlined per value, make the widest kernel's code long: 16
-// values for 1024 and 2048 points (2048^2 FP32 35.1 against 36.5, 4096^2 137 against 165; 8192^2
-// 690 against 687), and FP64 tiles of 2 rows at 2048 points (275 against 286). One-lane kernel
-// at its tuned variants: 256^2 FP64 8.1, FP32 8.2; 512^2 9.2, 8.5; 2048^2 59.3, 32.9; 4096^2
-// 260, 138 (packed, TMA); 8192^2 1375, 615 (packed, TMA); log 1024^2 22.5, 14.8, 2048^2 70.7,
-// 42.5, 4096^2 300, 174, 8192^2 FP32 780.
+// Row kernel with paired butterflies (power-of-two rows, whole tiles) and its passes' tables of
+// both sequences (one copy when they run the same radices). `tile`: the variant's rows per CTA,
+// or 0.
 template <class T>
 int pair_row_side(pfc_plan* h, int tile, std::vector<long double>& tw, FastRowSide& o) {
   const int lm = ilog2_exact(h->m);
-  if (lm < 6) return PFC_OK;   // (a tile of 32-point rows is less than a warp)
+  if (lm < kPairMinLog) return PFC_OK;
   const bool log = h->prob.model == PFC_MODEL_LOG;
-  int ee, rows;
-  if (sizeof(T) == 4) {
-    ee = lm <= 9 ? 8 : (log && lm <= 11) ? 16 : 32;
-    rows = (lm == 10 || (lm <= 9 && (tile >= 8 || (!tile && lm <= 7)))) ? 8 : 4;
-  } else {
-    ee = lm <= 9 ? 8 : 16;
-    rows = lm <= (log ? 10 : 11) ? 4 : 2;
-  }
+  const int ee = pair_ee(sizeof(T) == 8, lm, log), rows = pair_rows(sizeof(T) == 8, lm, log, tile);
   PairKernel k;
-  if (h->ny % rows || !PairInst<T>::row(lm, ee, rows, h->prob.model, &k)) return PFC_OK;
+  if (h->ny % rows || !PairInst<T>::row(lm, rows, h->prob.model, &k)) return PFC_OK;
   const std::vector<long double> root = unit_roots(h->m);
   std::vector<int> r = k.radices;
   build_pass_tables(h->m, r, root, tw, o.tw_a);

@@ -44,8 +44,29 @@ struct FastInst {
   static bool tables(int lg, std::vector<long double>& tw, int& offA, int& offB);
 };
 
-// Power-of-two row step kernels with paired butterflies (pfc_rowpair.cuh): 2^lg-point rows, ee
-// values per thread, `rows` rows a CTA (64- or 32-byte runs).
+// Power-of-two row step kernels with paired butterflies (pfc_rowpair.cuh) of 2^lg-point rows,
+// lg >= kPairMinLog (a tile of 32-point rows is less than a warp): values per thread, and rows
+// per CTA for a variant of `tile` rows (0: none asked for), by length, precision and model.
+// Rows of up to 512 points take 8 values a thread (the most threads; us per step on B200 with 8
+// / 16 values: 256^2 FP64 6.7 / 6.8, FP32 6.8 / 7.3, 512^2 8.0 / 8.5 and 7.4 / 8.7, 1024^2 log
+// 20.6 / 21.1 and 13.6 / 16.2), longer ones as many as 128 registers hold (2048^2 FP64 8 / 16
+// values 56.9 / 51.7, FP32 16 / 32 values 31.2 / 30.2, 8192^2 598 / 580). Tiles hold 64-byte
+// runs where a CTA of them fits an SM, and in FP32 32-byte ones for single plans of 256- and
+// 512-point rows, whose CTAs are few (512^2 7.4 against 7.7, 1024^2 log 13.6 against 14.2; a
+// batch of 24 512^2 plans prefers 8 rows, 41.3 against 43.1 us) and for 2048 points (121 against
+// 124). The log model's logarithms, inlined per value, make the widest kernel's code long: 16
+// values for 1024 and 2048 points (2048^2 FP32 35.1 against 36.5, 4096^2 137 against 165; 8192^2
+// 690 against 687), and FP64 tiles of 2 rows at 2048 points (275 against 286). One-lane kernel
+// at its tuned variants: 256^2 FP64 8.1, FP32 8.2; 512^2 9.2, 8.5; 2048^2 59.3, 32.9; 4096^2
+// 260, 138 (packed, TMA); 8192^2 1375, 615 (packed, TMA); log 1024^2 22.5, 14.8, 2048^2 70.7,
+// 42.5, 4096^2 300, 174, 8192^2 FP32 780.
+constexpr int kPairMinLog = 6;
+constexpr int pair_ee(bool fp64, int lg, bool log) { return lg <= 9 ? 8 : fp64 || (log && lg <= 11) ? 16 : 32; }
+constexpr int pair_rows(bool fp64, int lg, bool log, int tile) {
+  if (fp64) return lg <= (log ? 10 : 11) ? 4 : 2;
+  return lg == 10 || (lg <= 9 && (tile >= 8 || (!tile && lg <= 7))) ? 8 : 4;
+}
+
 struct PairKernel {
   void* fn = nullptr;
   int threads = 0;
@@ -54,7 +75,7 @@ struct PairKernel {
 };
 template <class T>
 struct PairInst {
-  static bool row(int lg, int ee, int rows, int model, PairKernel* out);
+  static bool row(int lg, int rows, int model, PairKernel* out);
 };
 
 // Register-resident step kernels for transforms of N = ODD * 2^k points, ODD = 3, 5, 7

@@ -179,7 +179,6 @@ row_step_pair(FastRowArgs<T> a) {
       [](cplx<T>& x) { x = mk(x.x + x.y, x.x - x.y); },
       [](cplx<T>& x) { x = T(2) * conj(x); });   // r_{M/2} = -i: S + U = 2 conj X
   {
-    using P0 = PairPass<T, M, EE, ROWS, false, 0>;
     dft_c<R0, true>(v);
     dft_c<R0, true>(v + R0);
     cplx<T>* p = buf + S::pad(t * R0) * ROWS;
@@ -189,7 +188,6 @@ row_step_pair(FastRowArgs<T> a) {
 #pragma unroll
     for (int q = 0; q < R0; ++q) q2[S::pad(q) * ROWS] = v[R0 + q];
     __syncthreads();
-    (void)sizeof(P0);
   }
   pair_mid<T, M, EE, ROWS, false, true, 1, NP - 1>(buf, v, t, a.twA);
   {

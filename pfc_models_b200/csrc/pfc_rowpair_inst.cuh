@@ -1,6 +1,6 @@
 // Definitions of PairInst (pfc_registry.h): included by the .cu file of each precision.
 #pragma once
-#include <cmath>
+#include <type_traits>
 
 #include "pfc_registry.h"
 #include "pfc_rowpair.cuh"
@@ -9,24 +9,17 @@ namespace pfc {
 
 namespace pair_detail {
 
-template <class T, int EE, int ROWS, int L>
-constexpr bool fits() {
-  // two passes or more; registers of a CTA within an SM's, its exchange buffer within 200 KB
-  constexpr int threads = ROWS * (1 << L) / EE;
-  if constexpr ((1 << L) < 2 * EE || threads < 32 || threads > 1024) return false;
-  else
-    return threads * PairMinBlocks<T, EE, threads>::regs <= 65536 &&
-           (size_t)PairSeq<(1 << L), EE>::SLOTS * ROWS * sizeof(cplx<T>) <= 200 * 1024;
-}
-
-template <class T, int EE, int ROWS, int L>
-bool row_l(int lg, int model, PairKernel* out) {
+// The kernels that pair_rows can ask for, with pair_ee's values per thread.
+template <class T, int ROWS, int MODEL, int L>
+bool row_l(int lg, PairKernel* out) {
+  constexpr bool fp64 = sizeof(T) == 8, log = MODEL == kModelLog;
   if constexpr (L <= kFastMaxLogRow) {
-    if (lg != L) return row_l<T, EE, ROWS, L + 1>(lg, model, out);
-    if constexpr (fits<T, EE, ROWS, L>()) {
+    if (lg != L) return row_l<T, ROWS, MODEL, L + 1>(lg, out);
+    if constexpr (pair_rows(fp64, L, log, 4) == ROWS || pair_rows(fp64, L, log, 8) == ROWS) {
+      constexpr int EE = pair_ee(fp64, L, log);
       using S = PairSeq<(1 << L), EE>;
-      out->fn = model == kModelLog ? (void*)row_step_pair<T, (1 << L), EE, ROWS, kModelLog>
-                                   : (void*)row_step_pair<T, (1 << L), EE, ROWS, kModelStd>;
+      static_assert(ROWS * S::TPF * PairMinBlocks<T, EE, ROWS * S::TPF>::regs <= 65536, "a CTA's registers");
+      out->fn = (void*)row_step_pair<T, (1 << L), EE, ROWS, MODEL>;
       out->threads = ROWS * S::TPF;
       out->smem = (size_t)S::SLOTS * ROWS * sizeof(cplx<T>);
       out->radices.clear();
@@ -40,18 +33,17 @@ bool row_l(int lg, int model, PairKernel* out) {
 }  // namespace pair_detail
 
 template <class T>
-bool PairInst<T>::row(int lg, int ee, int rows, int model, PairKernel* out) {
+bool PairInst<T>::row(int lg, int rows, int model, PairKernel* out) {
   using namespace pair_detail;
-  constexpr int RB = sizeof(T) == 4 ? 8 : 4;   // rows of a 64-byte run
-  if (lg < kFastMinLog || (rows != RB && rows != RB / 2)) return false;
-  auto pick = [&](auto e) {
-    constexpr int EE = decltype(e)::value;
-    return rows == RB ? row_l<T, EE, RB, kFastMinLog>(lg, model, out) : row_l<T, EE, RB / 2, kFastMinLog>(lg, model, out);
+  if (lg < kPairMinLog) return false;
+  auto pick = [&](auto r) {
+    constexpr int ROWS = decltype(r)::value;
+    return model == kModelLog ? row_l<T, ROWS, kModelLog, kPairMinLog>(lg, out)
+                              : row_l<T, ROWS, kModelStd, kPairMinLog>(lg, out);
   };
-  if (ee == 8) return pick(std::integral_constant<int, 8>{});
-  if (ee == 16) return pick(std::integral_constant<int, 16>{});
-  if constexpr (sizeof(T) == 4)
-    if (ee == 32) return pick(std::integral_constant<int, 32>{});
+  constexpr int RB = sizeof(T) == 4 ? 8 : 4;   // rows of a 64-byte run
+  if (rows == RB) return pick(std::integral_constant<int, RB>{});
+  if (rows == RB / 2) return pick(std::integral_constant<int, RB / 2>{});
   return false;
 }
 
