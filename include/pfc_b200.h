@@ -369,7 +369,7 @@ int pfc_abi_version(void);
  * OptimizeM (:332-373) sets M = (N(max) - N(min)) / (max - min), N(x) = g x^2 + x^3 + ln x,
  * and rebuilds the ETD1 coefficients of beta (q0^2 + lap)^2 + eps + M; the update is
  * phi_hat' = A_M phi_hat + B_M (Gamma lap (N_hat - M phi_hat) + lap V_hat) with the clamped
- * log (:524-577). The decision, M and the rebuild run on the device, stream-ordered. */
+ * log (:524-577). The decision, M and the rebuild run in the step's row and column kernels. */
 
 /* Replaces _ExternalPotential.SetPotential / SetGaussianDipolePotential /
  * SetPotential_alongX / SetDoubleVacancyAlongX_TanhPotential (models/logpfc_extv/

@@ -157,7 +157,8 @@ class Plan:
                 _lib.PATH_FAST_MIXED: "fast_mixed"}[v.value]
 
     def variant(self):
-        """{"ee_row", "ee_col", "row_tile", "fast"} of the step kernels this plan uses."""
+        """{"ee_row", "ee_col", "row_tile", "fast"} of the step kernels this plan uses
+        (row_tile 16 | rows: the row kernel with paired butterflies)."""
         o = (ctypes.c_int32 * 4)()
         _lib.check(self.lib.pfc_plan_variant(self.handle, o))
         return dict(zip(("ee_row", "ee_col", "row_tile", "fast"), list(o)))
@@ -576,10 +577,11 @@ class QueueBatch(Batch):
     """The same lockstep stepping as `Batch` in one persistent, cooperative launch per
     block of steps over a device list of work items (a row or column tile of one member at
     one step; pfc_queue_*), each item waiting only for the tiles of its own member that it
-    needs. Members must be stdPFC plans on the one-lane power-of-two kernels with the
-    values per thread the work-queue kernel is built with (`queue_kernels(nx, ny,
-    precision)` gives a kernel choice that has them), sides 64 .. 1024. Results are bit
-    for bit those of stepping each plan alone."""
+    needs. Members must be stdPFC plans on the power-of-two kernels with the values per
+    thread the work-queue kernel is built with (`queue_kernels(nx, ny, precision)` gives a
+    kernel choice that has them), sides 64 .. 1024. The work-queue kernel runs the one-lane
+    kernels: results are bit for bit those of stepping alone a plan made with
+    `queue_kernels`, and agree within rounding with one whose rows run the paired kernel."""
 
     def __init__(self, items):
         self.items = list(items)

@@ -14,7 +14,9 @@ package or the cache already holds). Results are cached as JSON, keyed
 by GPU name, grid, precision and model, in the file named by $PFC_TUNE_CACHE
 (default ~/.cache/pfc_models_b200/tune.json). `Simulation(kernels="auto")` looks
 a grid up there first, then in the table measured on B200 that ships with the
-package (tuned_b200.json), and otherwise uses the precision's defaults.
+package (tuned_b200.json), and otherwise uses the precision's defaults. Beside what it names,
+a choice found this way lets the plan take the row kernel with paired butterflies and, on
+odd-factor sides, the run-time kernel of a pass where that is faster.
 """
 from __future__ import annotations
 
