@@ -111,8 +111,10 @@ def run_points(points, steps, precision="fp32", block=1000, device=None, settle=
         if engine == "queue":
             variant = queue_kernels(p.n, p.n, precision)
         else:
-            # the kernel variant measured for batches of this box size, if there is one
-            variant = tune.lookup(p.n, p.n, _PRECISIONS[precision], _lib.MODEL_STD, batched=True) or "auto"
+            # the kernel variant measured for batches of this box size, if there is one (else
+            # the plan's own; FP32: the one-lane row kernel of its default, see tune.lookup)
+            variant = tune.lookup(p.n, p.n, _PRECISIONS[precision], _lib.MODEL_STD, batched=True) or \
+                ({"ee_row": 32} if _PRECISIONS[precision] == _lib.FP32_MIXED else "auto")
         sim = stdpfc.BuildB200_Simulation(prm, stdpfc.Build2DGeometry(p.n, p.n, p.lx, p.ly), precision=precision,
                                           device=device, kernels=variant)
         sim.State.n[...] = initial_field(p)

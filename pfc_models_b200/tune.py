@@ -74,7 +74,13 @@ def lookup(nx, ny, precision, model, device_name=None, batched=False):
     """The cached variant {"ee_row", "ee_col", "row_tile", "col_cta", "pdl"} for this
     grid, or None.
     `batched`: prefer the variant measured for many plans stepped as one batch (the
-    single-plan choice favours latency, a batch is throughput-bound)."""
+    single-plan choice favours latency, a batch is throughput-bound).
+
+    A choice for an FP32 batch is a plain variant, which runs the row kernel it names. A sweep's
+    members lie up to the limit of stability, where a state leaves through a transition that
+    rounding sets off: with the paired kernel's other order of summation single elements of a
+    128^2 .. 512^2 member moved by 8e-4 of the field's rms within 400 steps (other FP32 runs: up
+    to 5e-5), so a batch's results would depend on the kernel."""
     if device_name is None:
         try:
             device_name = _device_name()
@@ -86,7 +92,8 @@ def lookup(nx, ny, precision, model, device_name=None, batched=False):
         for path in (cache_path(), PACKAGED):
             e = _load(path).get(key)
             if e:
-                return _lib.TunedVariant({k: int(e.get(k) or 0) for k in VARIANT_KEYS})
+                v = {k: int(e.get(k) or 0) for k in VARIANT_KEYS}
+                return v if batched and precision == _lib.FP32_MIXED else _lib.TunedVariant(v)
     return None
 
 

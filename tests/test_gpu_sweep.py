@@ -58,3 +58,33 @@ def test_points_next_to_the_tangent_agree(both):
                 assert abs(q["F"] - p["F"]) < 1e-6 and abs(q["mu"] - p["mu"]) < 1e-5, p["index"]
                 n += 1
     assert n >= 6
+
+
+def test_fp32_members_keep_the_results_of_the_kernels_they_name():
+    """Crystals started within half a percent of the liquid's limit of stability leave their
+    state through a transition that rounding sets off: an FP32 batch's members on the choice that
+    tune.lookup gives equal, bit for bit after 400 steps, members on the one-lane row kernel with
+    the values per thread the sweep's boxes have always had."""
+    import torch
+    from pfc_models_b200 import _lib, stdpfc, tune
+    from pfc_models_b200.simulation import Batch
+    if torch.cuda.get_device_name() != "NVIDIA B200":
+        pytest.skip("the shipped table is for B200")
+    sims = []
+    for (n, mx, my), ee, r, factor in zip(sweep.BOXES, (8, 8, 16), (-0.30, -0.35, -0.41), (1.004, 1.002, 1.001)):
+        p = sweep.SweepPoint(0, r, -np.sqrt(-r / 3) * factor, n, mx, my, "crystal")
+        f = sweep.initial_field(p) + 0.01 * np.random.default_rng(n).uniform(-1, 1, (n, n))
+        prm = stdpfc.BuildStdPFCModelParameters(Gamma=1.0, beta=1.0, q0=1.0, epsilon=r, g=0.0, dt=sweep.DT)
+        for kernels in (tune.lookup(n, n, _lib.FP32_MIXED, _lib.MODEL_STD, batched=True),
+                        {"ee_row": ee, "ee_col": 8, "row_tile": 4}):
+            s = stdpfc.BuildB200_Simulation(prm, stdpfc.Build2DGeometry(n, n, p.lx, p.ly), precision="fp32",
+                                            kernels=kernels)
+            s.State.n[...] = f
+            sims.append(s)
+    b = Batch(sims)
+    b.step(400)
+    for a, ref in zip(sims[::2], sims[1::2]):
+        assert np.array_equal(a.State.n.get(), ref.State.n.get()), a.plan.shape
+    b.close()
+    for s in sims:
+        s.plan.close()

@@ -114,3 +114,14 @@ def test_refine_keeps_defaults_unless_clearly_faster(monkeypatch):
     # a grid the fast kernels do not cover keeps the defaults
     monkeypatch.setattr(tune, "_time_blocks", lambda *a, **k: (None, None))
     assert tune.refine(96, 96, "fp32", "std", base) == {"col_cta": 0, "pdl": 0}
+
+
+def test_fp32_batch_choice_names_its_row_kernel(tmp_path, monkeypatch):
+    """A choice for an FP32 batch is a plain variant (the row kernel it names runs); the others
+    let the plan pair its rows."""
+    monkeypatch.setenv("PFC_TUNE_CACHE", str(tmp_path / "none.json"))
+    for n in (128, 256, 512, 2048):      # (2048^2 has no batch entry: the single plan's)
+        kw = dict(device_name="NVIDIA B200", batched=True)
+        assert type(tune.lookup(n, n, _lib.FP32_MIXED, _lib.MODEL_STD, **kw)) is dict
+        assert type(tune.lookup(n, n, _lib.FP64_PLAIN, _lib.MODEL_STD, **kw)) is _lib.TunedVariant
+    assert type(tune.lookup(512, 512, _lib.FP32_MIXED, _lib.MODEL_STD, device_name="NVIDIA B200")) is _lib.TunedVariant
