@@ -505,7 +505,8 @@ __global__ void __launch_bounds__(LB, MINB) row_kernel(RowArgs<T> a) {
   if (MODE == kRowReduce) {
     // sums of: raw value (mean), free-energy polynomial, nonlinear mu
     const double mean = dev ? a_scal[kScalMean] : 0.0;
-    const double eps = a.epsilon, g = a.g;
+    const double eps = a.batch ? a.red[blockIdx.y].epsilon : a.epsilon, g = a.g;
+    double* partials = a.partials + (a.batch ? (size_t)blockIdx.y * a.partials_stride : 0);
     KSum acc[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
     if (valid) {
       for (int j = lt; j < m; j += tpf) {
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(LB, MINB) row_kernel(RowArgs<T> a) {
         for (int h = 0; h < 2; ++h) row_reduce_add<MODEL>(acc, mean, vv[h], eps, g, a.clamp, a.min_phi, a.min_log);
       }
     }
-    block_reduce_store<3>(acc, a.partials + 6 * blockIdx.x);
+    block_reduce_store<3>(acc, partials + 6 * blockIdx.x);
   }
 }
 

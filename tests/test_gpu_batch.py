@@ -261,3 +261,16 @@ def test_time_advances_as_single_steps_round():
     for _ in range(1000):
         want += dt
     assert _advanced(t, dt, 1000) == want and _advanced(t, dt, 1) == t + dt
+
+
+@pytest.mark.parametrize("precision,nx,ny", [("fp64", 16384, 6), ("fp64", 12288, 4), ("fp32", 32768, 4)])
+def test_batch_reduce_of_rows_in_one_buffer(precision, nx, ny):
+    """Rows too long for two buffers of shared memory reduce in the one-buffer row kernel: its
+    sums too belong to the plan of the grid row, with that plan's epsilon, bit for bit each
+    plan's own reduction."""
+    sims = [_std_sim(nx, ny, eps, -0.2 - 0.05 * i, precision, seed=i) for i, eps in enumerate((-0.3, -0.15, -0.45))]
+    b = Batch(sims)
+    for n in (0, 3):
+        b.step(n)
+        assert [tuple(r) for r in b.reduce()] == [s.Reduce() for s in sims], n
+    b.close()
