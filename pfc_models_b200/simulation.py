@@ -552,7 +552,16 @@ class Batch:
         return out.cpu().numpy()
 
     def _reduce_call(self, out):
-        _lib.check(self.lib.pfc_batch_reduce(self.handle, _ptr(out), _stream_ptr(self.torch, self.device)))
+        # the batch's launches read every plan's buffers: a closed plan refuses by itself (and a
+        # closed batch, whose tables are gone, leaves its plans to reduce one by one)
+        if self.handle.value and all(p.handle.value for p in self.plans):
+            _lib.check(self.lib.pfc_batch_reduce(self.handle, _ptr(out), _stream_ptr(self.torch, self.device)))
+        else:
+            self._reduce_each(out)
+
+    def _reduce_each(self, out):
+        for i, p in enumerate(self.plans):
+            p.reduce(out[i])
 
     @property
     def classes(self):
@@ -599,9 +608,7 @@ class QueueBatch(Batch):
     def _step_call(self, nsteps):
         _lib.check(self.lib.pfc_queue_step(self.handle, nsteps, _stream_ptr(self.torch, self.device)))
 
-    def _reduce_call(self, out):
-        for i, p in enumerate(self.plans):
-            p.reduce(out[i])
+    _reduce_call = Batch._reduce_each
 
     def status(self):
         """Status bits of the launches so far (synchronises): 0, or STATUS_TIMEOUT when a
