@@ -119,50 +119,6 @@ __device__ inline void block_minmax_store(double lo, double hi, double* out) {
   }
 }
 
-// Natural logarithm in FP64 without branches, so that the logarithms of a thread's values
-// overlap (the library function's special-case branches ran them one after another, 270 cycles
-// each: a 28 x 24 cell 2.75 -> 2.61 us a step, 256^2 log FP64 9.5 -> 8.9, 2048^2 64.9 -> 63.8).
-// x = 2^e (1 + f) with 1 + f in [sqrt(1/2), sqrt(2)); with s = f / (2 + f) the series of atanh gives
-// log(1 + f) = 2 (s + s^3/3 + s^5/5 + ...) = f - s (f - R), R = 2 (s^2/3 + s^4/5 + ...), in which f
-// is exact and the rounded part is at most f^2 / 2. |s| <= 0.1716: eleven terms leave 2e-18.
-// The division is a reciprocal estimate, two Newton steps and one correction of the quotient.
-// Against 80-bit values over 80 million arguments of all magnitudes: at most 0.96 ulp, 0.19 on
-// average; zero, negative, infinite, NaN and subnormal arguments as log().
-__device__ __forceinline__ double log_series(double x) {
-  const bool sub = x < 2.2250738585072014e-308;
-  const double xs = sub ? x * 18014398509481984.0 : x;   // 2^54
-  const long long bits = __double_as_longlong(xs);
-  // exponent such that the significand lies in [sqrt(1/2), sqrt(2)): subtract the bits of sqrt(1/2)
-  const int hi = (int)(bits >> 32) - 0x3fe6a09e;
-  const int e = hi >> 20;
-  const double m = __longlong_as_double(bits - ((long long)e << 52));
-  const double ef = (double)(e - (sub ? 54 : 0));
-  const double f = m - 1.0, d = m + 1.0;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
-  r = fma(r, fma(-d, r, 1.0), r);
-  double s = f * r;
-  s = fma(r, fma(-d, s, f), s);
-  const double z = s * s, w = z * z;
-  // R / z by even and odd terms
-  double a = fma(w, 0.08695652173913043, 0.10526315789473684);    // 2/23, 2/19
-  double b = fma(w, 0.09523809523809523, 0.11764705882352941);    // 2/21, 2/17
-  a = fma(w, a, 0.13333333333333333);                             // 2/15
-  b = fma(w, b, 0.15384615384615385);                             // 2/13
-  a = fma(w, a, 0.18181818181818182);                             // 2/11
-  b = fma(w, b, 0.2222222222222222);                              // 2/9
-  a = fma(w, a, 0.2857142857142857);                              // 2/7
-  b = fma(w, b, 0.4);                                             // 2/5
-  a = fma(w, a, 0.6666666666666666);                              // 2/3
-  const double R = z * fma(z, b, a);
-  // ln 2 in two parts, the first with 20 trailing zero bits (its product with e is exact)
-  const double c = s * (f - R);
-  double y = fma(ef, 0.6931471804855391, f - fma(ef, -7.440617110012397e-11, c));
-  y = x > 0.0 ? y : (x == 0.0 ? -INFINITY : NAN);
-  return (x < INFINITY) ? y : (x == INFINITY ? x : y);
-}
-
 // ---------------------------------------------------------------- nonlinearity
 // Plain FP64 form: the reference's expressions
 // (models/stdpfc/simulation.py:297, models/logpfc/simulation.py:296).
@@ -170,7 +126,7 @@ template <int MODEL>
 __device__ __forceinline__ double nonlin_plain(double n, double g, int clamp, double min_phi, double min_log) {
   const double n2 = n * n;
   double r = g * n2 + n2 * n;
-  if (MODEL == kModelLog) r += (clamp && !(n > min_phi)) ? min_log : log_series(n);
+  if (MODEL == kModelLog) r += (clamp && !(n > min_phi)) ? min_log : log(n);
   return r;
 }
 

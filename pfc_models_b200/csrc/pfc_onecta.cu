@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, MINB) onecta_step_kernel(Ro
 // tile) and as B[in][out] by the row products: the lane layouts of A (row lane / 4, column
 // lane % 4) and B (row lane % 4, column lane / 4) make the two the same table.
 // A 28 x 24 step needs 224 products, 900 cycles of an SM's FP64 rate (one m8n8k4 per 16 cycles
-// and scheduler); it takes 3800 (5000 with the log model's logarithms), now bound by the
-// instruction chain of its four phases: 2.0 us std, 2.6 us log, where the passes above take
+// and scheduler); it takes 3800 (5200 with the log model's logarithms), now bound by the
+// instruction chain of its four phases: 2.0 us std, 2.75 us log, where the passes above take
 // 6.0 and 6.7. tcgen05 has no FP64 form, so this is the FP64 tensor path of the chip.
 __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
