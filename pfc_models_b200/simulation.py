@@ -44,10 +44,22 @@ def _ptr(t):
 
 
 def _advanced(t, dt, nsteps):
-    """t after `nsteps` additions of dt, rounded one by one as a TimeStep loop rounds them."""
-    a = np.full(nsteps + 1, dt, dtype=np.float64)
-    a[0] = t
-    return np.add.accumulate(a)[-1]
+    """t after `nsteps` additions of dt, rounded one by one (and of the type) as a TimeStep loop
+    has them, in constant memory."""
+    t = t + dt
+    nsteps -= 1
+    if type(t) not in (float, np.float64):   # a caller's own number: its own addition
+        for _ in range(nsteps):
+            t += dt
+        return t
+    kind = type(t)
+    a = np.full(min(nsteps, 1 << 16) + 1, dt, dtype=np.float64)
+    while nsteps:
+        k = min(nsteps, len(a) - 1)
+        a[0] = t
+        t = np.add.accumulate(a[:k + 1])[-1]
+        nsteps -= k
+    return kind(t)
 
 
 class ModelParameters:
@@ -535,9 +547,13 @@ class Batch:
             if isinstance(s, Simulation):
                 s._version += 1
                 s._mu_current = False
-                key = (s.State.t, s.Model.dt)
+                t, dt = s.State.t, s.Model.dt
+                if not {type(t), type(dt)} <= {float, np.float64}:
+                    s.State.t = _advanced(t, dt, nsteps)
+                    continue
+                key = (type(t), t, type(dt), dt)
                 if key not in times:
-                    times[key] = _advanced(*key, nsteps)
+                    times[key] = _advanced(t, dt, nsteps)
                 s.State.t = times[key]
 
     def _step_call(self, nsteps):

@@ -67,3 +67,28 @@ def test_polycrystal_generator():
     assert 0 < changed.sum() <= 4 * np.pi * 144 + 50
     # the profile A (cos u cos v - cos(2v)/2) peaks at 0.75 A
     assert -0.3 + 0.7 * 0.5 < a[changed].max() <= -0.3 + 0.75 * 0.5 + 1e-12
+
+
+def test_time_of_a_block_of_steps():
+    """State.t after a block: a loop's additions bit for bit past one chunk, of the loop's type,
+    without memory that grows with the steps."""
+    import tracemalloc
+    from fractions import Fraction
+    from pfc_models_b200.simulation import _advanced
+
+    def loop(t, dt, n):
+        for _ in range(n):
+            t += dt
+        return t
+    for t, dt in ((np.float64(0.7), np.float64(0.1)), (0.0, 0.5), (0, np.float64(0.1)), (3, 2), (Fraction(1, 3), Fraction(1, 7)),
+                  (np.float32(0.1), 0.1), (-0.0, 0.0), (float("nan"), 0.1)):
+        for n in (1, 2, 1000):
+            got, want = _advanced(t, dt, n), loop(t, dt, n)
+            assert type(got) is type(want) and (got == want or want != want), (t, dt, n)
+    want = loop(0.7, 0.1, 3 * 65536 + 5)
+    assert _advanced(0.7, 0.1, 3 * 65536 + 5) == want
+    tracemalloc.start()
+    _advanced(np.float64(0), np.float64(0.1), 10 ** 7)
+    peak = tracemalloc.get_traced_memory()[1]
+    tracemalloc.stop()
+    assert peak < 4 << 20
