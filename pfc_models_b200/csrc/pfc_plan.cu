@@ -1040,8 +1040,10 @@ int setup_onecta(pfc_plan* h) {
     d.col_tab = tw + h->dense_col;
     d.g = ra.g; d.min_phi = ra.min_phi; d.min_log = ra.min_log; d.clamp = ra.clamp;
     d.scale = col_args<double>(h).scale;
-    cudaError_t e = dense_allow_smem(kOneCtaMaxSmem);
-    if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
+    if (bytes > 48 * 1024) {
+      cudaError_t e = dense_allow_smem(kOneCtaMaxSmem);
+      if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
+    }
     h->oc_smem = bytes;
     h->onecta = true;
     return PFC_OK;
