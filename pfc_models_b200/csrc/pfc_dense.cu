@@ -15,9 +15,14 @@
 // A fragment entry (out, in) is read as A[out][in] by the column products (out = rows of the
 // tile) and as B[in][out] by the row products: the lane layouts of A (row lane / 4, column
 // lane % 4) and B (row lane % 4, column lane / 4) make the two the same table.
+// A sum of n / 2 terms in a chain rounds more than an FFT's log n levels, most of all by the mean
+// density, which every partial sum would carry. So the step transforms n - nbar and N - N(nbar),
+// the mean being constant: its error against 80-bit values, pooled over 11 sizes and both models
+// after 1 and 10 steps, is 0.92 times that of the FFT passes (1.14 with the mean; two chains a sum
+// beside it would give 0.90, and 3 % more time).
 // A 28 x 24 step needs 224 products, 900 cycles of an SM's FP64 rate (one m8n8k4 per 16 cycles
-// and scheduler); it takes 3800 (5200 with the log model's logarithms), now bound by the
-// instruction chain of its four phases: 2.0 us std, 2.75 us log, where the FFT passes take
+// and scheduler); it takes 4000 (5600 with the log model's logarithms), bound by the
+// instruction chain of its four phases: 2.1 us std, 2.9 us log, where the FFT passes take
 // 6.0 and 6.7. tcgen05 has no FP64 form, so this is the FP64 tensor path of the chip.
 // A translation unit of its own: the driver loads a unit's code at its first kernel's first use,
 // and the unrolled butterflies of pfc_onecta.cu are megabytes of it (24 ms of a process's first
@@ -61,6 +66,8 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
   const int lr = lane >> 2, lc = lane & 3;
   const double s2 = 2.0 * a.scale;
+  // the mean density, which every step keeps (the k = 0 mode's coefficients are zero), and its N
+  const double nbar = a.scale * P[0][0].x, nref = nonlin_plain<MODEL>(nbar, a.g, a.clamp, a.min_phi, a.min_log);
 
   // (the areas' padding is only ever multiplied by zero entries of the tables: any finite value)
   for (int i = tid; i < a.size_a + a.size_b; i += nth) areaA[i] = 0.0;
@@ -72,7 +79,7 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
     const double2 w = W[i];
     S[i] = P[0][i];
     if (k == 0) {
-      wre[y] = 2.0 * w.x;
+      wre[y] = 2.0 * (w.x - nbar);
       wre[m * ys + y] = 2.0 * w.y;
     } else {
       wre[k * ys + y] = 2.0 * w.x;
@@ -104,7 +111,7 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
   };
   for (long long step = 0; step < nsteps; ++step) {
     const bool last = step == nsteps - 1;
-    // ---- 1: n = C - S at x, C + S at nx - x; N of both; folded over x
+    // ---- 1: n - nbar = C - S at x, C + S at nx - x; N - nref of both; folded over x
     row_tiles([&](int y, int tx) {
       double c0 = 0.0, c1 = 0.0, s0 = 0.0, s1 = 0.0;
       const double *pr = wre + lc * ys + y + lr, *pi = wim + lc * ys + y + lr;
@@ -115,10 +122,10 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
         dmma(c0, c1, pr[4 * q * ys], w.x);
         dmma(s0, s1, pi[4 * q * ys], w.y);
       }
-      const double p0 = nonlin_plain<MODEL>(c0 - s0, a.g, a.clamp, a.min_phi, a.min_log);
-      const double q0 = nonlin_plain<MODEL>(c0 + s0, a.g, a.clamp, a.min_phi, a.min_log);
-      const double p1 = nonlin_plain<MODEL>(c1 - s1, a.g, a.clamp, a.min_phi, a.min_log);
-      const double q1 = nonlin_plain<MODEL>(c1 + s1, a.g, a.clamp, a.min_phi, a.min_log);
+      const double p0 = nonlin_plain<MODEL>(nbar + (c0 - s0), a.g, a.clamp, a.min_phi, a.min_log) - nref;
+      const double q0 = nonlin_plain<MODEL>(nbar + (c0 + s0), a.g, a.clamp, a.min_phi, a.min_log) - nref;
+      const double p1 = nonlin_plain<MODEL>(nbar + (c1 - s1), a.g, a.clamp, a.min_phi, a.min_log) - nref;
+      const double q1 = nonlin_plain<MODEL>(nbar + (c1 + s1), a.g, a.clamp, a.min_phi, a.min_log) - nref;
       const int x = tx * 8 + 2 * lc, yy = y + lr;
       if (yy < ny) {
         if (x <= m) {
@@ -132,7 +139,7 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
       }
     });
     __syncthreads();
-    // ---- 2: V[k] = C - i S
+    // ---- 2: V[k] = C - i S (of N - nref: V[0] lacks nx nref)
     row_tiles([&](int y, int tx) {
       double c0 = 0.0, c1 = 0.0, s0 = 0.0, s1 = 0.0;
       const double *pe = ne + lc * ys + y + lr, *po = no + lc * ys + y + lr;
@@ -148,7 +155,7 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
         if (yy >= ny || k > m) return;
         if (k == 0 || k == m) {
           rv[(k == 0 ? 0 : ys) + yy] = re;
-          if (last) V[2 * yy + (k == 0 ? 0 : 1)] = re;
+          if (last) V[2 * yy + (k == 0 ? 0 : 1)] = k == 0 ? re + 2.0 * m * nref : re;
         } else {
           rv[2 * k * ys + yy] = re;
           rv[(2 * k + 1) * ys + yy] = im;
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
           p_new[k * ny + ky] = o;
           p_new[k * ny + kyp] = op;
         }
-        xe[2 * k * ks + ky] = ok.x + okp.x;
+        xe[2 * k * ks + ky] = k == 0 && ky == 0 ? 0.0 : ok.x + okp.x;   // (without the mean)
         xe[(2 * k + 1) * ks + ky] = ok.y + okp.y;
         xo[2 * k * ks + ky] = ok.x - okp.x;
         xo[(2 * k + 1) * ks + ky] = ok.y - okp.y;
@@ -224,11 +231,19 @@ __global__ void __launch_bounds__(kOneCtaMaxThreads, 2) onecta_dense_kernel(Dens
       }
       const int y = tk * 8 + lr, k = (c >> 1) + lc;
       if (y <= h && k < m) {
+        // (column 0 is rounded with the mean, as it is kept in memory: where a launch ends is no
+        // matter then)
         auto put = [&](int yy, double re, double im) {
-          wre[k * ys + yy] = s2 * re;
-          if (k == 0) wre[m * ys + yy] = s2 * im;
-          else wim[k * ys + yy] = s2 * im;
-          if (last) W[k * ny + yy] = make_double2(a.scale * re, a.scale * im);
+          double w = a.scale * re;
+          if (k == 0) {
+            w += nbar;
+            wre[yy] = 2.0 * (w - nbar);
+            wre[m * ys + yy] = s2 * im;
+          } else {
+            wre[k * ys + yy] = s2 * re;
+            wim[k * ys + yy] = s2 * im;
+          }
+          if (last) W[k * ny + yy] = make_double2(w, a.scale * im);
         };
         put(y, p0 - q1, p1 + q0);
         if (y != 0 && ny - y != y) put(ny - y, p0 + q1, p1 - q0);
