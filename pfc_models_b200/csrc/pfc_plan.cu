@@ -648,22 +648,36 @@ int setup_tma(pfc_plan* h) {
   return raise_smem_limit(h->fast_row_fn, h->fr_smem);
 }
 
-// Odd-factor columns whose register-resident kernel (few threads holding ODD values each) is
-// slower than the run-time one. B200, column pass with its events, register-resident against
-// run-time, us: 3 x 128 FP32 20.3 / 12.7, FP64 14.0 / 11.8, 3 x 256 16.6 / 18.7 and 14.7 / 18.7;
-// 5 x 128 16.8 / 14.2 and 20.5 / 12.5, 5 x 256 22.4 / 25.9 and 33.9 / 29.1, 5 x 512 52.9 / 72.1 and
-// 90.2 / 96.3; 7 x 128 20.1 / 14.7 and 27.0 / 19.2, 7 x 256 26.7 / 34.8 and 58.7 / 46.4.
-bool short_odd_column(int ny, bool fp32) {
+// Odd-factor columns whose register-resident kernel (few threads holding ODD values each, a long
+// chain that a few CTAs take as long for as many) is slower than the run-time one, whose time
+// grows with the points sooner. B200, column pass with its events, register-resident / run-time,
+// us, at m columns: FP32 3 x 128 m = 512 19.9 / 11.9, 2048 22.2 / 20.3, 4096 25.4 / 26.9; 5 x 64
+// 2048 20.3 / 17.8, 4096 23.8 / 27.8; 5 x 128 512 16.7 / 12.8, 640 16.6 / 18.5, 2048 20.9 / 30.3;
+// 7 x 64 2048 24.6 / 20.6, 4096 28.8 / 32.2; 7 x 128 1024 21.8 / 21.3, 2048 26.6 / 34.2. FP64
+// 3 x 128 512 14.1 / 11.8, 640 14.1 / 16.3; 3 x 64 1024 13.3 / 10.9, 2048 14.0 / 15.0; 5 x 64 2048
+// 20.3 / 18.7, 4096 30.4 / 31.0; 5 x 128 512 20.4 / 17.7, 640 20.5 / 21.0; 5 x 256 256 20.7 / 14.7,
+// 512 20.6 / 22.0; 7 x 32 to 7 x 256 up to 4096 201 / 152. Longer ones from 3 x 256 (FP64 5 x 512,
+// 7 x 512) on keep the register-resident kernel at every width.
+bool short_odd_column(int ny, int m, bool fp32) {
   int odd = ny;
   while (odd % 2 == 0) odd /= 2;
   const int p2 = ny / odd;
-  return odd == 3 ? p2 < 256 : odd == 5 ? p2 < (fp32 ? 256 : 512) : p2 < (fp32 ? 256 : 512);
+  const long long points = (long long)m * ny;
+  if (p2 >= (odd == 3 || fp32 ? 256 : 512)) return false;
+  if (odd == 7 && !fp32) return true;
+  if (odd == 3 && !fp32) return points <= 3 << 16;
+  return points <= (odd == 5 && p2 >= 128 ? 3 << 17 : 1 << 20);
 }
 
-// FP64 rows of 7 x 32 points and more: 28 complex doubles a thread leave too few threads. Row
-// pass, register-resident against run-time, us: 7 x 32 21.2 / 13.0, 7 x 64 26.0 / 17.5, 7 x 128
-// 74 / 60 (7 x 16 16.5 / 11.4 keeps the register-resident kernel beside its columns).
-bool long_odd7_row(int m, bool fp32) { return !fp32 && m % 7 == 0 && m >= 7 * 32; }
+// FP64 rows of 7 x 32 points and more: 28 complex doubles a thread leave too few threads, until
+// the grid fills them. Row pass, register-resident / run-time, us, at ny rows: 7 x 32 ny = 2048
+// 25.1 / 18.9, 4096 29.0 / 31.5; 7 x 64 2048 31.1 / 27.1, 4096 47.6 / 47.8; 7 x 128 256 27.1 /
+// 16.0, 4096 124 / 112; 7 x 256 256 33.1 / 22.2, 512 34.5 / 37.3, 1024 71.5 / 69.7, 4096 227 / 260;
+// 7 x 512 96 39.4 / 27.0, 256 40.4 / 46.1, 2048 266 / 339.
+bool long_odd7_row(int m, int ny, bool fp32) {
+  if (fp32 || m % 7 || m < 7 * 32) return false;
+  return m == 7 * 128 || (long long)m * ny <= (m == 7 * 64 ? 1 << 20 : 1 << 19);
+}
 
 // Values per thread of a power-of-two column kernel by its length, as the tuned entries of
 // that length have it.
@@ -744,8 +758,8 @@ int setup_fast(pfc_plan* h, std::vector<long double>& tw) {
   // short odd-factor columns, and a power-of-two side's kernel beside a side without one.
   const bool row2 = ilog2_exact(h->m) >= 0, col2 = ilog2_exact(h->ny) >= 0;
   const bool split = (fr & PFC_EE_PAIRED) && !onecta_fits(h);
-  const bool drop_row = split && r.ok && !row2 && long_odd7_row(h->m, sizeof(T) == 4);
-  const bool drop_col = split && c.ok && !c.packed && !col2 && short_odd_column(h->ny, sizeof(T) == 4);
+  const bool drop_row = split && r.ok && !row2 && long_odd7_row(h->m, h->ny, sizeof(T) == 4);
+  const bool drop_col = split && c.ok && !c.packed && !col2 && short_odd_column(h->ny, h->m, sizeof(T) == 4);
   r.ok = r.ok && !drop_row;
   c.ok = c.ok && !drop_col;
   if (!r.ok && !c.ok) return PFC_OK;   // run-time kernels
