@@ -57,3 +57,19 @@ def test_runtime_kernels_at_sequence_edges(nx, ny, model, precision):
     assert mean_mu == pytest.approx(o.mu_per_site(), rel=ftol, abs=ftol)
     assert mean_n == pytest.approx(float(o.n.mean()), rel=1e-12)
     sim.plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ny", [(4, 2), (8, 30), (16, 75), (32, 392), (26, 33), (990, 5)])
+def test_upload_of_narrow_fields(nx, ny, precision):
+    """Tiles of up to 32 rows, the last one partly filled: a field comes back as it was uploaded,
+    within the rounding of a forward and an inverse transform."""
+    from pfc_models_b200 import stdpfc
+    prm = stdpfc.BuildStdPFCModelParameters(Gamma=1.0, beta=1.0, q0=1.0, epsilon=-0.25, g=0.0, dt=0.5)
+    sim = stdpfc.BuildB200_Simulation(prm, stdpfc.Build2DGeometry(nx, ny, 0.78 * nx, 0.78 * ny), precision=precision)
+    f = np.random.default_rng(nx * ny).uniform(-1, 1, (ny, nx))
+    sim.State.n[...] = f
+    eps = np.finfo(np.float64 if precision == "fp64" else np.float32).eps
+    assert np.abs(sim.State.n.get() - f).max() <= 4 * eps * np.log2(nx * ny)
+    sim.plan.close()
