@@ -33,7 +33,7 @@ template <class T, int MODE>
 void* pick_col(int rset) {
   // (the Parseval and export modes transform nothing)
   if constexpr (MODE == kColParseval || MODE == kColExport) {
-    return (void*)col_kernel<T, MODE, kRadixPow2, 256>;
+    return (void*)col_kernel<T, MODE, kRadixPow2, kParThreads>;
   } else {
     switch (rset) {
       case kRadixPow2: return (void*)mixed_col_kernel<T, MODE, kRadixPow2>;

@@ -19,6 +19,8 @@ namespace pfc {
 constexpr int kRadixPow2Big = 2;
 constexpr int kRadixSmallBig = 6;
 constexpr size_t kMixedSmem = 200 * 1024;
+// most threads of a Parseval or export CTA, which hold one column of 4096 points or more
+constexpr int kParThreads = 512;
 
 // log2 sizes of the power-of-two step kernels: row transforms of M = nx/2 points,
 // column transforms of ny points
