@@ -244,7 +244,7 @@ int pfc_batch_reduce(pfc_batch* batch, double* out, void* stream);
 
 int pfc_batch_destroy(pfc_batch* batch);
 
-/* Kernel launches issued by pfc_batch_step and pfc_batch_reduce so far; number of classes. */
+/* Kernel launches issued by pfc_batch_step so far; number of classes. */
 int64_t pfc_batch_launch_count(pfc_batch* batch);
 int pfc_batch_classes(pfc_batch* batch);
 

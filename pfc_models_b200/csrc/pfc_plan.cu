@@ -1356,7 +1356,6 @@ int do_batch_reduce(pfc_batch* b, double* out, cudaStream_t s) {
     }
     const BatchBufs* table = c.table[h->cur];
     const int stride = (int)reduce_partials(h);
-    const long long own = h->launches;   // (the launches are the batch's)
     RowArgs<T> ra = row_args<T>(h);
     ra.partials = c.partials;
     ra.batch = table; ra.red = c.red; ra.partials_stride = stride;
@@ -1367,9 +1366,7 @@ int do_batch_reduce(pfc_batch* b, double* out, cudaStream_t s) {
     ca.partials = colp;
     ca.batch = table; ca.red = c.red; ca.partials_stride = stride;
     rc = launch_col<T, kColParseval>(h, ca, s, n);
-    h->launches = own;
     if (rc) return rc;
-    b->launches += 3;
     finalize_reduce_kernel<<<n, merge_threads(std::max(h->row_grid, h->par_grid)), 0, s>>>(
         c.partials, h->row_grid, colp, h->par_grid, stride, nullptr, BatchReduce{}, table, c.red, c.slot,
         1.0 / ((double)h->nx * (double)h->ny), h->fp32 ? 1 : 0, out);

@@ -274,14 +274,3 @@ def test_batch_reduce_of_rows_in_one_buffer(precision, nx, ny):
         b.step(n)
         assert [tuple(r) for r in b.reduce()] == [s.Reduce() for s in sims], n
     b.close()
-
-
-def test_batch_reduce_counts_its_launches_on_the_batch():
-    """A batched reduction's three launches a class are the batch's, not its first plan's."""
-    sims = [_std_sim(nx, 64, -0.3, -0.25, "fp64", seed=i) for i, nx in enumerate((64, 128, 64))]
-    b = Batch(sims)
-    own, before = [s.plan.launches() for s in sims], b.launches()
-    b.reduce()
-    assert b.launches() - before == 3 * b.classes == 6
-    assert [s.plan.launches() for s in sims] == own
-    b.close()
