@@ -239,7 +239,8 @@ int pfc_batch_create(pfc_plan* const* plans, int32_t count, pfc_batch** out);
  * states were set, mod 2), else PFC_E_STATE. Stream-ordered. */
 int pfc_batch_step(pfc_batch* batch, int64_t nsteps, void* stream);
 /* pfc_reduce of every plan, in the order of pfc_batch_create: out holds 3 doubles per plan in
- * device memory. Three launches per class; each plan's values equal its pfc_reduce bit for bit. */
+ * device memory. Three launches per class, counted on its first plan; each plan's values equal its
+ * pfc_reduce bit for bit. */
 int pfc_batch_reduce(pfc_batch* batch, double* out, void* stream);
 
 int pfc_batch_destroy(pfc_batch* batch);

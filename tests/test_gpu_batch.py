@@ -274,3 +274,15 @@ def test_batch_reduce_of_rows_in_one_buffer(precision, nx, ny):
         b.step(n)
         assert [tuple(r) for r in b.reduce()] == [s.Reduce() for s in sims], n
     b.close()
+
+
+def test_batch_reduce_counts_all_its_launches():
+    """A batched reduction's three launches a class count as its first plan's (the batch's own
+    count is that of its steps)."""
+    sims = [_std_sim(nx, 64, -0.3, -0.25, "fp64", seed=i) for i, nx in enumerate((64, 128, 64))]
+    b = Batch(sims)
+    own, before = [s.plan.launches() for s in sims], b.launches()
+    b.reduce()
+    assert [s.plan.launches() - n for s, n in zip(sims, own)] == [3, 3, 0]
+    assert b.launches() == before and b.classes == 2
+    b.close()
