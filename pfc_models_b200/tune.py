@@ -16,7 +16,8 @@ by GPU name, grid, precision and model, in the file named by $PFC_TUNE_CACHE
 a grid up there first, then in the table measured on B200 that ships with the
 package (tuned_b200.json), and otherwise uses the precision's defaults. Beside what it names,
 a choice found this way lets the plan take the row kernel with paired butterflies and, on
-odd-factor sides, the run-time kernel of a pass where that is faster.
+odd-factor sides, the run-time kernel of a pass where that is faster, unless the kernels that it
+names were timed faster than those ("named").
 """
 from __future__ import annotations
 
@@ -93,7 +94,8 @@ def lookup(nx, ny, precision, model, device_name=None, batched=False):
             e = _load(path).get(key)
             if e:
                 v = {k: int(e.get(k) or 0) for k in VARIANT_KEYS}
-                return v if batched and precision == _lib.FP32_MIXED else _lib.TunedVariant(v)
+                named = e.get("named") or (batched and precision == _lib.FP32_MIXED)
+                return v if named else _lib.TunedVariant(v)
     return None
 
 
@@ -194,7 +196,7 @@ def tune(nx, ny, precision="fp32", model="std", steps=20, warmup=3, save=True, p
              "row_us": row_us, "col_us": col_us,
              "rows_us": {f"{tag(a)}{b}/{c}/{d}": u for (a, b, c, d), u in sorted(rows.items())},
              "cols_us": {f"{tag(a)}{b}": u for (a, b), u in sorted(col_avg.items())}}
-    entry.update(refine(nx, ny, precision, model, entry))
+    entry.update(choose(nx, ny, precision, model, entry))
     if save:
         _store(path or cache_path(), _key(_device_name(), nx, ny, prec,
                                           _lib.MODEL_LOG if model == "log" else _lib.MODEL_STD), entry)
@@ -257,7 +259,7 @@ def _tune_batch(nx, ny, precision, model, steps, warmup, save, path, batch):
     entry = {"ee_row": ee_r, "ee_col": ee_c, "row_tile": tile, "batch": batch, "step_us": us,
              "row_us": None, "col_us": None,
              "steps_us": {f"{a}/{b}/{c}": u for (a, b, c), u in sorted(timed.items())}}
-    entry.update(refine(nx, ny, precision, model, entry, batch=batch))
+    entry.update(choose(nx, ny, precision, model, entry, batch=batch))
     if save:
         _store(path or cache_path(), _key(_device_name(), nx, ny, prec,
                                           _lib.MODEL_LOG if model == "log" else _lib.MODEL_STD, True), entry)
@@ -308,11 +310,29 @@ def _time_blocks(nx, ny, precision, model, variant, batch, steps=320, skip=None,
             s.plan.close()
 
 
-def refine(nx, ny, precision, model, base, batch=1, min_gain=0.01):
-    """Second stage: columns per CTA of the column kernel and programmatic dependent
+def choose(nx, ny, precision, model, base, batch=1, min_gain=0.01):
+    """Second stage of a choice found by `lookup`: `refine` with the kernels that the plan takes
+    by itself (paired rows, passes mixed) and with the ones that `base` names. The named ones
+    ("named": 1 in the entry) where they are at least `min_gain` faster; FP32 batches run only
+    those."""
+    if batch > 1 and precision == "fp32":
+        return refine(nx, ny, precision, model, base, batch, min_gain, kind=dict)
+    own = refine(nx, ny, precision, model, base, batch, min_gain)
+    named = refine(nx, ny, precision, model, base, batch, min_gain, kind=dict)
+
+    def us(r):
+        return r["refine_us"][f"{r['col_cta']}/{r['pdl']}"] if "refine_us" in r else math.inf
+    if us(named) < (1 - min_gain) * us(own):
+        return dict(named, named=1)
+    return dict(own, named=0)
+
+
+def refine(nx, ny, precision, model, base, batch=1, min_gain=0.01, kind=_lib.TunedVariant):
+    """Columns per CTA of the column kernel and programmatic dependent
     launch for the row/column variant in `base`, timed over whole steps. Returns
     {"col_cta", "pdl", "refine_us"}; keeps the defaults (0, 0) unless a choice is at
-    least `min_gain` faster than they are."""
+    least `min_gain` faster than they are. `kind`: what the plan is given, a TunedVariant (its own
+    kernels) or a dict (the named ones)."""
     v0 = {k: int(base.get(k) or 0) for k in ("ee_row", "ee_col", "row_tile", "packed", "tma")}
     timed, seen = {}, set()
     # sides with an odd factor: the register-resident kernels hold a fixed number of values
@@ -322,7 +342,7 @@ def refine(nx, ny, precision, model, base, batch=1, min_gain=0.01):
         generic_us, _ = _time_blocks(nx, ny, precision, model, {"generic": 1}, batch, fast=False)
     for cc in (0,) + COL_CTA_CHOICES:
         for pdl in (0, 1, 2):   # 2: the column kernel only
-            us, threads = _time_blocks(nx, ny, precision, model, _lib.TunedVariant(v0, col_cta=cc, pdl=pdl), batch,
+            us, threads = _time_blocks(nx, ny, precision, model, kind(v0, col_cta=cc, pdl=pdl), batch,
                                        skip=lambda th: (th, pdl) in seen)
             if threads is None:
                 return {"col_cta": 0, "pdl": 0}
@@ -352,7 +372,7 @@ def refine_table(path_in, device_name, steps=320):
         nx, ny = (int(v) for v in parts[1].split("x"))
         batch = int(e.get("batch") or 1) if len(parts) > 4 and parts[4] == "batch" else 1
         e = dict(e)
-        e.update(refine(nx, ny, parts[2], parts[3], e, batch=batch))
+        e.update(choose(nx, ny, parts[2], parts[3], e, batch=batch))
         d[key] = e
         print(json.dumps({key: {k: e.get(k) for k in VARIANT_KEYS + ("refine_us",)}}), flush=True)
     return d

@@ -125,3 +125,31 @@ def test_fp32_batch_choice_names_its_row_kernel(tmp_path, monkeypatch):
         assert type(tune.lookup(n, n, _lib.FP32_MIXED, _lib.MODEL_STD, **kw)) is dict
         assert type(tune.lookup(n, n, _lib.FP64_PLAIN, _lib.MODEL_STD, **kw)) is _lib.TunedVariant
     assert type(tune.lookup(512, 512, _lib.FP32_MIXED, _lib.MODEL_STD, device_name="NVIDIA B200")) is _lib.TunedVariant
+
+
+def test_choose_lets_named_kernels_win(monkeypatch, tmp_path):
+    """The second stage times the plan's own kernels (a TunedVariant) and the named ones (a dict);
+    where the named ones are at least 1 % faster the entry says so, and lookup returns a dict,
+    which the plan runs as named. FP32 batches time only the named ones. Faked timings."""
+    seen, gain = [], {}
+
+    def fake(nx, ny, precision, model, variant, batch, steps=320, skip=None, fast=True):
+        seen.append(type(variant))
+        th = 128 * (1 + variant.get("col_cta", 0))
+        if skip is not None and skip(th):
+            return None, th
+        return (10.0 if type(variant) is _lib.TunedVariant else gain["named"]) + variant.get("col_cta", 0), th
+    monkeypatch.setattr(tune, "_time_blocks", fake)
+    base = {"ee_row": 8, "ee_col": 0, "row_tile": 8}
+    path = str(tmp_path / "t.json")
+    monkeypatch.setenv("PFC_TUNE_CACHE", path)
+    for us, named, kind in ((9.95, 0, _lib.TunedVariant), (9.8, 1, dict)):
+        gain["named"] = us
+        e = tune.choose(512, 512, "fp64", "std", base)
+        assert e["named"] == named and (e["col_cta"], e["pdl"]) == (0, 0)
+        tune._store(path, tune._key("X", 512, 512, _lib.FP64_PLAIN, _lib.MODEL_STD), dict(base, **e))
+        v = tune.lookup(512, 512, _lib.FP64_PLAIN, _lib.MODEL_STD, device_name="X")
+        assert type(v) is kind and v["ee_row"] == 8
+    seen.clear()
+    tune.choose(512, 512, "fp32", "std", base, batch=24)
+    assert set(seen) == {dict}
