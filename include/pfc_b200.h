@@ -177,8 +177,8 @@ int pfc_plan_info(pfc_plan* plan, int64_t* out16);
 /* OR-ed into a PFC_FLAG_ROW_EE value, or PFC_TILE_PAIRED into a PFC_FLAG_ROW_TILE value of 2, 4
  * or 8: on power-of-two rows the plan takes the row kernel with paired butterflies, at its own
  * values per thread, as it does when PFC_FLAG_ROW_EE and PFC_FLAG_ROW_TILE are 0. Where that
- * kernel does not apply (nx/2 not a power of two, ny not whole tiles), and for the work queue,
- * the rest of the variant counts. With PFC_EE_PAIRED the plan also mixes kernels by pass: short
+ * kernel does not apply (nx/2 not a power of two, ny not whole tiles), and for whether the work
+ * queue takes the plan, the rest of the variant counts. With PFC_EE_PAIRED the plan also mixes kernels by pass: short
  * odd-factor columns, and the side without a register-resident kernel beside a power-of-two one,
  * run the run-time kernels. */
 #define PFC_TILE_PAIRED 16

@@ -232,7 +232,7 @@ struct pfc_plan {
   bool packed = false;         // two-lane packed FP32 step kernels (pfc_pack_step.cuh) on either pass
   bool packed_row = false, packed_col = false;
   bool paired_row = false;     // row kernel with paired butterflies (pfc_rowpair.cuh)
-  FastRowSide one_row;         // the one-lane row kernel's shape, which the work-queue kernel runs
+  FastRowSide one_row;         // the one-lane row kernel's shape, by which the work queue takes a plan
   // log PFC with an external potential (PFC_FLAG_EXTV, pfc_extv.cu)
   bool extv = false;
   pfc::ExtvState* extv_st = nullptr;   // device
@@ -2262,7 +2262,7 @@ int queue_build(pfc_queue* q) {
     int c = 0;
     for (; c < (int)q->classes.size(); ++c) {
       const pfc_plan* r = q->plans[q->classes[c][0]];
-      if (r->one_row.fn == h->one_row.fn && r->fast_col_fn == h->fast_col_fn && r->one_row.rows == h->one_row.rows &&
+      if (r->one_row.fn == h->one_row.fn && r->paired_row == h->paired_row && r->fast_col_fn == h->fast_col_fn && r->one_row.rows == h->one_row.rows &&
           r->fc_threads == h->fc_threads && r->nx == h->nx && r->ny == h->ny && r->prob.g == h->prob.g &&
           r->prob.clamp_log == h->prob.clamp_log && r->prob.min_phi == h->prob.min_phi)
         break;
@@ -2277,13 +2277,26 @@ int queue_build(pfc_queue* q) {
     const std::vector<int>& mem = q->classes[c];
     const pfc_plan* r = q->plans[mem[0]];
     QueueClass<T>& k = host[c];
-    const FastRowSide& row = r->one_row;
+    // the plan's own row kernel: paired (its tables; a row's values do not depend on the tile) or one-lane
+    FastRowSide row = r->one_row;
+    k.paired = r->paired_row;
     k.row = fast_row_args<T>(r, nullptr);
+    if (r->paired_row) {
+      PairKernel pk;
+      row.rows = queue_pair_rows(sizeof(T) == 8, r->m);
+      if (!PairInst<T>::row(ilog2_exact(r->m), row.rows, PFC_MODEL_STD, &pk) || pk.threads > kQueueThreads ||
+          pk.smem > kQueueSmemMax)
+        return fail(PFC_E_ARG, "pfc_queue_create: no paired row body for rows of %d points", r->m);
+      row.threads = pk.threads;
+      row.smem = pk.smem;
+      row.grid = r->ny / row.rows;
+    } else {
+      k.row.twA = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_a;
+      k.row.twB = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_b;
+    }
     k.row.rows = row.rows;
     k.row.ld = row.ld;
     k.row.rows_log2 = ilog2_exact(row.rows);
-    k.row.twA = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_a;
-    k.row.twB = reinterpret_cast<const cplx<T>*>(r->tw) + row.tw_b;
     k.col = fast_col_args<T>(r, nullptr);
     k.row_log = ilog2_exact(r->m);
     k.col_log = ilog2_exact(r->ny);

@@ -2,8 +2,8 @@
 // by a block of steps in ONE persistent launch.
 //
 // The unit of work (an item) is one row tile or one column tile of one plan at one step,
-// the same tiles the step kernels of pfc_fast.cuh run as CTAs, through the same bodies
-// (row_step_body / col_step_body), so a plan stepped here computes bit for bit what its
+// the same tiles the step kernels run as CTAs, through the same bodies (row_step_body and
+// col_step_body of pfc_fast.cuh, row_pair_body of pfc_rowpair.cuh for plans with paired rows), so a plan stepped here computes bit for bit what its
 // own launches compute. An item's dependencies are the plan's own: its row tiles of step
 // s need all of its column tiles of step s - 1 (W, and V free to overwrite), its column
 // tiles of step s all of its row tiles of step s (V; n_hat of step s - 1 follows). Each
@@ -29,7 +29,8 @@
 // become ld.global.cg here (COHERENT = true); tables and coefficients, written before the
 // launch, keep their loads.
 #pragma once
-#include "pfc_fast.cuh"
+#include "pfc_rowpair.cuh"
+#include "pfc_registry.h"
 
 namespace pfc {
 
@@ -42,6 +43,12 @@ __host__ __device__ constexpr int queue_col_ee(bool fp64, int ny) { return fp64 
 // .. 1024 wide), columns of 64 .. 1024 points
 constexpr int kQueueMinLogRow = 5, kQueueMaxLogRow = 9, kQueueMinLogCol = 6, kQueueMaxLogCol = 10;
 constexpr int kQueueThreads = 256;
+// Rows per tile of the paired row body: 64-byte runs of W and V within kQueueThreads threads (a
+// row's values do not depend on its tile).
+__host__ __device__ constexpr int queue_pair_rows(bool fp64, int m) { return !fp64 && m <= 256 ? 8 : 4; }
+static_assert(pair_ee(false, kPairMinLog, false) == 8 && pair_ee(false, kQueueMaxLogRow, false) == 8 &&
+              pair_ee(true, kPairMinLog, false) == 8 && pair_ee(true, kQueueMaxLogRow, false) == 8,
+              "the paired body's 8 values a thread fit the queue kernel's 64 registers");
 constexpr long long kQueueWaitLimit = 1LL << 20;   // polls (an L2 round trip and 64 ns each): about a second
 
 // One size class: plans of one grid and one step variant.
@@ -51,6 +58,7 @@ struct QueueClass {
   FastColArgs<T> col;
   const BatchBufs* table[2];   // the members' buffers, by the parity of the step
   int row_log, col_log;        // log2 of the row (M) and column (ny) transform lengths
+  int paired;                  // row pass with paired butterflies
   int row_threads, col_threads;
   int row_items, col_items;    // items of one member's pass
   int row_group, col_group;    // consecutive tiles per item (a member's tiles = items x group)
@@ -106,6 +114,12 @@ __device__ __noinline__ void queue_row_body(const QueueClass<T>* C, const BatchB
   row_step_body<T, M, queue_row_ee(sizeof(T) == 8, M), kModelStd, true>(C->row, table, tile, local,
                                                                         C->row_threads, NoSync{});
 }
+template <class T, int M>
+__device__ __noinline__ void queue_pair_body(const QueueClass<T>* C, const BatchBufs* table, int tile, int local) {
+  constexpr int ROWS = queue_pair_rows(sizeof(T) == 8, M);
+  static_assert(ROWS * (M / 8) <= kQueueThreads && ROWS * (M / 8) % 32 == 0, "whole warps of a queue CTA");
+  row_pair_body<T, M, 8, ROWS, kModelStd, true>(C->row, table, tile, local, NoSync{});
+}
 template <class T, int NY>
 __device__ __noinline__ void queue_col_body(const QueueClass<T>* C, const BatchBufs* table, int tile, int local) {
   constexpr int EE = queue_col_ee(sizeof(T) == 8, NY);
@@ -121,6 +135,12 @@ __device__ __forceinline__ void queue_row_item(const QueueClass<T>& C, const Bat
   if constexpr (L <= kQueueMaxLogRow) {
     if (C.row_log == L) {
       constexpr int M = 1 << L;
+      if constexpr (L >= kPairMinLog) {
+        if (C.paired) {
+          queue_pair_body<T, M>(&C, table, tile, local);
+          return;
+        }
+      }
       queue_row_body<T, M>(&C, table, tile, local);
       return;
     }

@@ -104,17 +104,25 @@ struct PairPass {
   }
 };
 
+// Barrier of the THREADS threads that run the body: the whole CTA in the step kernel, the first
+// ones (whole warps) of a work-queue CTA, on the named barrier of body_sync.
+template <int THREADS, bool QUEUE>
+__device__ __forceinline__ void pair_sync() {
+  if constexpr (QUEUE) asm volatile("bar.sync 15, %0;" ::"n"(THREADS) : "memory");
+  else __syncthreads();
+}
+
 // Passes [PA, PB) of a sequence in place through buf.
-template <class T, int N, int EE, int ROWS, bool SEQB, bool INV, int PA, int PB>
+template <class T, int N, int EE, int ROWS, bool SEQB, bool INV, bool QUEUE, int PA, int PB>
 __device__ __forceinline__ void pair_mid(cplx<T>* buf, cplx<T>* v, int t, const cplx<T>* __restrict__ tw) {
   if constexpr (PA < PB) {
     using P = PairPass<T, N, EE, ROWS, SEQB, PA>;
     P::load(buf, v, t);
-    __syncthreads();
+    pair_sync<ROWS * (N / EE), QUEUE>();
     P::template compute<INV>(v, t, tw);
     P::store(buf, v, t);
-    __syncthreads();
-    pair_mid<T, N, EE, ROWS, SEQB, INV, PA + 1, PB>(buf, v, t, tw);
+    pair_sync<ROWS * (N / EE), QUEUE>();
+    pair_mid<T, N, EE, ROWS, SEQB, INV, QUEUE, PA + 1, PB>(buf, v, t, tw);
   }
 }
 
@@ -136,38 +144,39 @@ __device__ __forceinline__ void pair_elements(cplx<T>* va, cplx<T>* vb, int t, F
   }
 }
 
-template <class T, int M, int EE, int ROWS, int MODEL>
-__global__ void __launch_bounds__(ROWS * (M / EE), PairMinBlocks<T, EE, ROWS * (M / EE)>::value)
-row_step_pair(FastRowArgs<T> a) {
+// Row tile `tile` of member `member` on the first ROWS * M / EE threads of the CTA. QUEUE: in the
+// work-queue kernel, where other CTAs of the launch write W (coherent loads).
+template <class T, int M, int EE, int ROWS, int MODEL, bool QUEUE, class Sync>
+__device__ __forceinline__ void row_pair_body(const FastRowArgs<T>& a, const BatchBufs* batch, int tile, int member,
+                                              Sync sync) {
   using S = PairSeq<M, EE>;
-  constexpr int R0 = S::R0, NR = M / R0, NP = S::NP;
+  constexpr int R0 = S::R0, NR = M / R0, NP = S::NP, THREADS = ROWS * S::TPF;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int r = threadIdx.x & (ROWS - 1), t = threadIdx.x / ROWS;
   cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw) + r;
   const size_t ny = a.ny;
-  const int y = blockIdx.x * ROWS + r;
+  const int y = tile * ROWS + r;
   const cplx<T>* gin = a.in;
   cplx<T>* gout = a.out;
   const double* scal = a.scal;
-  if (a.batch) {
-    const BatchBufs& b = a.batch[blockIdx.y];
+  if (batch) {
+    const BatchBufs& b = batch[member];
     gin = static_cast<const cplx<T>*>(b.w);
     gout = static_cast<cplx<T>*>(b.v);
     scal = b.scal;
   }
   const int jb = t == 0 ? NR / 2 : NR - t;   // the second butterfly
 
-  pdl_wait();
-  pdl_trigger();
+  sync();   // W is the previous column pass's output
 
   cplx<T> v[EE];
   {
     const cplx<T>* pa = gin + t * ny + y;
     const cplx<T>* pb = gin + jb * ny + y;
 #pragma unroll
-    for (int q = 0; q < R0; ++q) v[q] = ldsc(pa + q * (NR * ny));
+    for (int q = 0; q < R0; ++q) v[q] = ld_field<QUEUE>(pa + q * (NR * ny));
 #pragma unroll
-    for (int q = 0; q < R0; ++q) v[R0 + q] = ldsc(pb + q * (NR * ny));
+    for (int q = 0; q < R0; ++q) v[R0 + q] = ld_field<QUEUE>(pb + q * (NR * ny));
   }
   // Z[k] = S + U, Z[M - k] = conj(S - U), S = X[k] + conj X[M-k], U = i conj(r_k) (X[k] - conj X[M-k])
   pair_elements<R0, NR>(v, v + R0, t,
@@ -187,9 +196,9 @@ row_step_pair(FastRowArgs<T> a) {
     for (int q = 0; q < R0; ++q) p[S::pad(q) * ROWS] = v[q];
 #pragma unroll
     for (int q = 0; q < R0; ++q) q2[S::pad(q) * ROWS] = v[R0 + q];
-    __syncthreads();
+    pair_sync<THREADS, QUEUE>();
   }
-  pair_mid<T, M, EE, ROWS, false, true, 1, NP - 1>(buf, v, t, a.twA);
+  pair_mid<T, M, EE, ROWS, false, true, QUEUE, 1, NP - 1>(buf, v, t, a.twA);
   {
     using PL = PairPass<T, M, EE, ROWS, false, NP - 1>;
     PL::load(buf, v, t);
@@ -213,11 +222,11 @@ row_step_pair(FastRowArgs<T> a) {
   {
     using Q0 = PairPass<T, M, EE, ROWS, true, 0>;
     Q0::template compute<false>(v, t, a.twB);
-    __syncthreads();   // every thread has read the last exchange
+    pair_sync<THREADS, QUEUE>();   // every thread has read the last exchange
     Q0::store(buf, v, t);
-    __syncthreads();
+    pair_sync<THREADS, QUEUE>();
   }
-  pair_mid<T, M, EE, ROWS, true, false, 1, NP - 1>(buf, v, t, a.twB);
+  pair_mid<T, M, EE, ROWS, true, false, QUEUE, 1, NP - 1>(buf, v, t, a.twB);
   {
     using QL = PairPass<T, M, EE, ROWS, true, NP - 1>;
     static_assert(QL::R == R0 && QL::NS == NR, "sequence B ends with the radix that A begins with");
@@ -249,6 +258,12 @@ row_step_pair(FastRowArgs<T> a) {
 #pragma unroll
     for (int q = 0; q < R0; ++q) pb[q * (NR * ny)] = v[R0 + q];
   }
+}
+
+template <class T, int M, int EE, int ROWS, int MODEL>
+__global__ void __launch_bounds__(ROWS * (M / EE), PairMinBlocks<T, EE, ROWS * (M / EE)>::value)
+row_step_pair(FastRowArgs<T> a) {
+  row_pair_body<T, M, EE, ROWS, MODEL, false>(a, a.batch, blockIdx.x, blockIdx.y, PdlSync{});
 }
 
 }  // namespace pfc

@@ -604,9 +604,8 @@ class QueueBatch(Batch):
     one step; pfc_queue_*), each item waiting only for the tiles of its own member that it
     needs. Members must be stdPFC plans on the power-of-two kernels with the values per
     thread the work-queue kernel is built with (`queue_kernels(nx, ny, precision)` gives a
-    kernel choice that has them), sides 64 .. 1024. The work-queue kernel runs the one-lane
-    kernels: results are bit for bit those of stepping alone a plan made with
-    `queue_kernels`, and agree within rounding with one whose rows run the paired kernel."""
+    kernel choice that has them), sides 64 .. 1024. Results are bit for bit those of stepping
+    each plan alone: a member runs the row kernel that it runs by itself."""
 
     def __init__(self, items):
         self.items = list(items)

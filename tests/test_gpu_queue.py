@@ -129,3 +129,35 @@ def test_queue_wait_runs_out_and_reports():
     for s, r in zip(sims, ref):
         assert np.array_equal(_state(s), _state(r))
     q.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_queue_members_keep_the_row_kernel_they_choose(precision):
+    """Members whose plans chose their kernels run paired rows by themselves and in the queue:
+    bit for bit the same states, at every row length with a paired kernel, beside members on the
+    one-lane kernels of the same sizes."""
+    grids = [(nx, ny) for nx in (128, 256, 512, 1024) for ny in (64, 256)] + [(64, 128)]
+
+    def members():
+        out = []
+        for i, (nx, ny) in enumerate(grids):
+            one = queue_kernels(nx, ny, precision)
+            paired = {"ee_row": one["ee_row"], "ee_col": one["ee_col"], "row_tile": 16 | 4}
+            if nx == 64:   # (32-point rows have no paired kernel)
+                paired["row_tile"] = one["row_tile"]
+            for j, kernels in enumerate((paired, one)):
+                out.append(_sim(nx, ny, -0.3, -0.25, precision, 2 * i + j, kernels))
+        for n in (256, 512) if precision == "fp64" else ():   # (tuned choices the queue takes)
+            out.append(_sim(n, n, -0.3, -0.25, precision, 100 + n, "auto"))
+        return out
+    ref, sims = members(), members()
+    assert sum(bool(s.plan.variant()["row_tile"] & 16) for s in sims) >= 8
+    q = QueueBatch(sims)
+    for k in (1, 16, 33):
+        q.step(k)
+        for r in ref:
+            r.TimeSteps(k)
+    assert q.status() == 0
+    for a, b in zip(ref, sims):
+        assert np.array_equal(_state(a), _state(b)), (a.plan.shape, a.plan.variant())
+    q.close()
