@@ -160,3 +160,16 @@ def test_one_cta_transforms_against_oracle(model, nx, ny):
         lmu = float(np.max(np.abs(o.lin_mu)))
         assert np.linalg.norm(sim.mu.get() - mu) <= 1e-12 * (np.linalg.norm(mu) + lmu * np.linalg.norm(o.n)), n
         assert sim.CalculateFreeEnergy() == pytest.approx(o.free_energy(), rel=1e-12, abs=1e-13)
+
+
+# the FFT passes: rows or columns of a single pass, and sides with 11 and 13 (more products than a
+# dense plan's 800: 1972, 6840, 1008, 1360)
+FFT_GRIDS = [(8, 225), (450, 4), (26, 65), (130, 14)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", FFT_GRIDS)
+@pytest.mark.parametrize("model", ["std", "log"])
+def test_one_cta_fft_passes_against_oracle(model, nx, ny):
+    """As above, for the one-CTA step whose transforms are FFT passes."""
+    test_one_cta_transforms_against_oracle(model, nx, ny)
