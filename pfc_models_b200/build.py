@@ -28,7 +28,8 @@ SOURCES = ["pfc_plan.cu", "pfc_generic_f32.cu", "pfc_generic_f64.cu",
            "pfc_rowpair_f32.cu", "pfc_rowpair_f64.cu", "pfc_fastmix_f32.cu", "pfc_fastmix_f64.cu", "pfc_queue_f32.cu", "pfc_queue_f64.cu"]
 HEADERS = ["pfc_fft.cuh", "pfc_kernels.cuh", "pfc_fast.cuh", "pfc_small.cuh", "pfc_registry.h",
            "pfc_fast_inst.cuh", "pfc_generic_inst.cuh", "pfc_pack.cuh", "pfc_pack_step.cuh", "pfc_fastmix_inst.cuh",
-           "pfc_queue.cuh", "pfc_mixed.cuh", "pfc_extv.h", "pfc_rowpair.cuh", "pfc_rowpair_inst.cuh"]
+           "pfc_queue.cuh", "pfc_mixed.cuh", "pfc_extv.h", "pfc_rowpair.cuh", "pfc_rowpair_body.cuh",
+           "pfc_rowpair_inst.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC"]

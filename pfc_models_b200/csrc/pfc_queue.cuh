@@ -3,7 +3,7 @@
 //
 // The unit of work (an item) is one row tile or one column tile of one plan at one step,
 // the same tiles the step kernels run as CTAs, through the same bodies (row_step_body and
-// col_step_body of pfc_fast.cuh, row_pair_body of pfc_rowpair.cuh for plans with paired rows), so a plan stepped here computes bit for bit what its
+// col_step_body of pfc_fast.cuh, row_pair_queue of pfc_rowpair.cuh for plans with paired rows), so a plan stepped here computes bit for bit what its
 // own launches compute. An item's dependencies are the plan's own: its row tiles of step
 // s need all of its column tiles of step s - 1 (W, and V free to overwrite), its column
 // tiles of step s all of its row tiles of step s (V; n_hat of step s - 1 follows). Each
@@ -118,7 +118,7 @@ template <class T, int M>
 __device__ __noinline__ void queue_pair_body(const QueueClass<T>* C, const BatchBufs* table, int tile, int local) {
   constexpr int ROWS = queue_pair_rows(sizeof(T) == 8, M);
   static_assert(ROWS * (M / 8) <= kQueueThreads && ROWS * (M / 8) % 32 == 0, "whole warps of a queue CTA");
-  row_pair_body<T, M, 8, ROWS, kModelStd, true>(C->row, table, tile, local, NoSync{});
+  row_pair_queue<T, M, 8, ROWS, kModelStd>(C->row, table, tile, local);
 }
 template <class T, int NY>
 __device__ __noinline__ void queue_col_body(const QueueClass<T>* C, const BatchBufs* table, int tile, int local) {
