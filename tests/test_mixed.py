@@ -73,3 +73,12 @@ def test_upload_of_narrow_fields(nx, ny, precision):
     eps = np.finfo(np.float64 if precision == "fp64" else np.float32).eps
     assert np.abs(sim.State.n.get() - f).max() <= 4 * eps * np.log2(nx * ny)
     sim.plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(32, 16), (32, 45), (90, 16)])
+@pytest.mark.parametrize("model", ["std", "log"])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_sixteen_point_transforms(nx, ny, model, precision):
+    """Rows and columns of 16 points (two passes of radix 4) against the oracle, as above."""
+    test_runtime_kernels_at_sequence_edges(nx, ny, model, precision)
