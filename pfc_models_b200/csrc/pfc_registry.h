@@ -146,7 +146,7 @@ cudaError_t launch_onecta_step(const RowArgs<double>& ra, const ColArgs<double>&
                                int count, long long nsteps, int model, int rset, bool dense, int threads,
                                size_t smem, cudaStream_t stream);
 
-// The same step with dense transforms on the FP64 tensor cores (onecta_dense_kernel).
+// The same step with dense transforms on the FP64 tensor cores (pfc_dense.cu).
 struct DenseArgs {
   int m, ny, nyh;                  // half row length, column length, coefficients a column
   int tr, kr, tc, kc;              // 8-wide output tiles and 4-deep steps of the row and column matrices
@@ -162,7 +162,8 @@ int dense_products(const DenseArgs& a);                    // m8n8k4 products of
 // the square of the sides. B200, us a step, one cell / 296 cells in one batch, dense against
 // FFT passes: 28 x 24 (224 products) 2.0 / 2.8 against 6.0 / 6.3, 48 x 20 (512) 3.7 / 4.8
 // against 5.5 / 6.2, 30 x 50 (672) 4.2 / 5.9 against 6.4 / 7.6, 32 x 56 (932) 5.4 / 7.9
-// against 6.6 / 7.8 and for the log model 7.4 / 10.6 against 8.0 / 9.6.
+// against 6.6 / 7.8 and for the log model 7.4 / 10.6 against 8.0 / 9.6 (dense before it took the mean
+// out of its transforms, 0.13 us a step more on 28 x 24).
 constexpr int kDenseMaxProducts = 800;
 // appends the (w cos, w sin) fragments of length n; root = exp(-2 pi i k / n), k < n
 void dense_table(int n, const std::vector<long double>& root, std::vector<long double>& tw);
