@@ -1,4 +1,4 @@
-// Whole-grid step kernel for the smallest FP64 mixed-radix cells: the step of pfc_onecta.cu (one
+// Whole-grid step kernel for the smallest FP64 mixed-radix cells: the step of pfc_onecta.cuh (one
 // CTA per plan, `nsteps` steps a launch) with every transform as a small FP64 matrix product on
 // the tensor cores (mma.sync m8n8k4). At these lengths the chain of FFT phases, not its
 // arithmetic, is the step: the FFT passes run 12 % of the issue slots, waiting at barriers for
@@ -24,9 +24,8 @@
 // and scheduler); it takes 4000 (5600 with the log model's logarithms), bound by the
 // instruction chain of its four phases: 2.1 us std, 2.9 us log, where the FFT passes take
 // 6.0 and 6.7. tcgen05 has no FP64 form, so this is the FP64 tensor path of the chip.
-// A translation unit of its own: the driver loads a unit's code at its first kernel's first use,
-// and the unrolled butterflies of pfc_onecta.cu are megabytes of it (24 ms of a process's first
-// 28 x 24 plan).
+// A translation unit of its own: the driver loads a unit's code as one, at its first kernel's first
+// use, and a large unit slowly (24 ms of a process's first 28 x 24 plan with pfc_onecta.cuh's kernels).
 #include <algorithm>
 #include <cmath>
 

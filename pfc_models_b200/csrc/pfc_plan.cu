@@ -255,7 +255,7 @@ struct pfc_plan {
   // CUDA graphs of kGraphBlock steps and of one step, one per starting ping-pong parity
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   cudaGraphExec_t graph1[2] = {nullptr, nullptr};
-  // small FP64 mixed-radix grids: whole steps in one CTA (pfc_onecta.cu), reading this
+  // small FP64 mixed-radix grids: whole steps in one CTA (pfc_onecta.cuh), reading this
   // plan's buffers from a one-entry table per parity of cur
   bool onecta = false;
   int oc_threads = 0, oc_rset = kRadixPow2, oc_sms = 0;
@@ -1036,7 +1036,7 @@ int setup_onecta(pfc_plan* h) {
   const size_t smem = onecta_smem_bytes(h->m, h->ny, h->row_ld, h->col_ld);
   if (!onecta_fits(h)) return PFC_OK;
   if (smem > 48 * 1024) {
-    cudaError_t e = onecta_allow_smem(kOneCtaMaxSmem);
+    cudaError_t e = onecta_allow_smem(kOneCtaMaxSmem, h->prob.model, rset);
     if (e != cudaSuccess) return fail(PFC_E_CUDA, "pfc_plan_create: one-CTA shared memory: %s", cudaGetErrorString(e));
   }
   for (int p = 0; p < 2; ++p) {

@@ -131,7 +131,7 @@ cudaError_t launch_defect_screen(const double* field, const double* spec, int nx
                                  double* partials, double* out4, cudaStream_t stream);
 int diagnose_partials_needed();
 
-// Whole-grid step kernel for small FP64 mixed-radix grids (pfc_onecta.cu): one CTA per
+// Whole-grid step kernel for small FP64 mixed-radix grids (pfc_onecta.cuh): one CTA per
 // plan runs nsteps steps with the grid in shared memory; `table` holds the plans'
 // buffers (BatchBufs) at the starting parity, `count` entries.
 template <class T> struct RowArgs;
@@ -140,7 +140,10 @@ struct BatchBufs;
 constexpr int kOneCtaMaxThreads = 256;
 constexpr size_t kOneCtaMaxSmem = 96 * 1024;   // two CTAs per SM
 size_t onecta_smem_bytes(int m, int ny, int row_ld, int col_ld);
-cudaError_t onecta_allow_smem(size_t bytes);     // raises the kernels' dynamic shared memory limit
+// raises the dynamic shared memory limit of a model's and radix set's kernels
+cudaError_t onecta_allow_smem(size_t bytes, int model, int rset);
+// the kernel at one CTA an SM, or (dense) at two
+template <int MODEL, int RSET> struct OnectaInst { static void* kernel(bool dense); };
 bool onecta_supported(int rset);
 cudaError_t launch_onecta_step(const RowArgs<double>& ra, const ColArgs<double>& ca, const BatchBufs* table,
                                int count, long long nsteps, int model, int rset, bool dense, int threads,
